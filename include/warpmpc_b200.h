@@ -349,6 +349,18 @@ int wmpc_stream_schedule_host(const wmpc_pattern_desc* desc, const float* rho, c
                               int32_t n_primal, int32_t units, int32_t cols, int32_t rel, int32_t funits,
                               int32_t offload, int32_t* out, int64_t out_capacity, int64_t* out_words);
 
+/* Host-only export of the band form's tables (the persistent solve's form for
+ * patterns that factor into short subtrees and one band-like chain; used to
+ * verify them on the CPU).  rho/rhoinv and n_primal as above.
+ * WMPC_ERR_UNSUPPORTED (with the reason) where the pattern has no such form.
+ * out: [n, n_prim, n_pre, T, T4, units, n_chunks, chunk_cols, n_yr, nb, blen,
+ * chunk_bytes, item_bytes, n_far, n_rows, n_pad]
+ * col_word[T4] chunk[4 n_chunks] far_ptr[n_chunks] far[n_far]
+ * item[2 n_pre + nb + T] rec[32 n_rows] rec_off[n_rows] iter_off[n]
+ * param_off[n] lpos[nnz_l] lpos2[nnz_l] dpos[n] pad[n_pad]. */
+int wmpc_band_tables_host(const wmpc_pattern_desc* desc, const float* rho, const float* rhoinv, int32_t n_primal,
+                          int32_t* out, int64_t out_capacity, int64_t* out_words);
+
 /* Profiling (no counterpart in the reference, which times with wall
  * clocks around jax.block_until_ready).  Between begin and end the library
  * records a CUDA event pair on the launching stream around every launch of
@@ -363,7 +375,7 @@ int wmpc_profile_end(float* dominant_ms, int32_t* dominant_launches, int64_t* to
  * reference. */
 int wmpc_profile_select(int32_t channel);
 /* The last streaming ADMM launch of this process (no counterpart in the
- * reference): info = {schedule form (0 none yet, 1 plain, 2 frontier),
+ * reference): info = {schedule form (0 none yet, 1 plain, 2 frontier, 3 band),
  * CTAs per SM, grid size, dynamic shared memory bytes}. */
 int wmpc_stream_last_launch(int32_t info[4]);
 /* Kernels launched by this library since load (or the last profile_begin). */

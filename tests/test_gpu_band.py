@@ -1,0 +1,158 @@
+"""The band form of the persistent solve on the GPU (warpmpc_b200/csrc/band.cu).
+
+The arithmetic and its order are the other forms': iterates equal the float32
+oracle's bit for bit, and checked or rho-adapting solves equal the streaming
+form's, iteration and refactorization counts included.  ``WMPC_STREAM_BAND=1``
+runs it wherever its tables can be built, 0 nowhere.
+"""
+
+import numpy as np
+import pytest
+
+from oracle import osqp_ref
+from warpmpc_b200 import native, problems
+from warpmpc_b200.jax_osqp import OSQPSettings, compile_osqp, solve_classes
+
+pytestmark = pytest.mark.gpu
+
+
+def _dev(*arrays):
+    import torch
+
+    return [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in arrays]
+
+
+def _compile(monkeypatch, plan, band):
+    monkeypatch.setenv("WMPC_STREAM_BAND", str(band))
+    comp = compile_osqp(plan, np.float32, qdldl_backend="cuda", transpose_work=True, mode="persistent")
+    monkeypatch.delenv("WMPC_STREAM_BAND")
+    return comp
+
+
+def _warm(plan, batch, seed):
+    rng = np.random.default_rng(seed)
+    return [(rng.standard_normal((batch, k)) * 0.1).astype(np.float32) for k in (plan.n, plan.m, plan.m)]
+
+
+SHORT = problems.MPCClass("short quadrotor", 12, 4, 2, 10.0, 2.0, 1.0, "quadrotor")
+
+
+@pytest.mark.parametrize("cls,batch,ctas", [(problems.SMALL, 1, 1), (problems.SMALL, 9500, 2), (problems.CARTPOLE, 97, 1),
+                                            (problems.CARTPOLE, 4801, 1), (SHORT, 33, 1), (problems.QUADROTOR, 32, 1),
+                                            (problems.QUADROTOR, 4801, 1)], ids=lambda v: getattr(v, "name", str(v)))
+def test_band_form_bitexact(cuda_device, monkeypatch, cls, batch, ctas):
+    """One lane, whole and partial tiles, one and two CTAs per SM, 8- and
+    16-row windows, a chain of a few chunks, several tiles per CTA."""
+    from oracle.cpu_baseline import CpuOSQP
+
+    b = problems.make_batch(cls, batch, seed=31)
+    plan = problems.make_plan(b)
+    comp = _compile(monkeypatch, plan, 1)
+    got = comp.engine.solve(*_dev(b.p_values, b.a_values, b.q, b.l, b.u))
+    launch = native.stream_last_launch()
+    assert launch["form"] == "band" and launch["ctas_per_sm"] == ctas, launch
+    ref = CpuOSQP(plan).solve(b.p_values, b.a_values, b.q, b.l, b.u)
+    for name, g, r in zip(("x", "z", "y"), got[:3], ref[:3]):
+        np.testing.assert_array_equal(g.cpu().numpy(), r, err_msg=name)
+    assert not np.any(comp.engine.last_status.cpu().numpy() & 8)
+
+
+@pytest.mark.parametrize("cls", [problems.SMALL, problems.QUADROTOR], ids=lambda c: c.name)
+def test_band_form_warm_start_shared_matrices(cuda_device, monkeypatch, cls):
+    b = problems.make_batch(cls, 45, seed=6)
+    plan = problems.make_plan(b)
+    comp = _compile(monkeypatch, plan, 1)
+    warm = _warm(plan, 45, 2)
+    args = (b.p_values[:1], b.a_values[:1], b.q, b.l, b.u)
+    got = comp.engine.solve(*_dev(*args), warm=tuple(_dev(*warm)))
+    ref = osqp_ref.solve_warm_start(plan, *args, *warm)
+    for g, r in zip(got[:3], ref[:3]):
+        np.testing.assert_array_equal(g.cpu().numpy(), r)
+
+
+@pytest.mark.parametrize("cls,batch", [(problems.SMALL, 40), (problems.SMALL, 9500), (problems.CARTPOLE, 5300),
+                                       (problems.QUADROTOR, 70)], ids=lambda v: getattr(v, "name", str(v)))
+def test_band_form_termination_checks(cuda_device, monkeypatch, cls, batch):
+    """Tiles that stop early, and what follows them on the same CTA."""
+    b = problems.make_batch(cls, batch, seed=3)
+    plan = problems.make_plan(b, OSQPSettings(**{**problems.DEFAULT_SETTINGS, "max_iter": 60}))
+    band, plain = _compile(monkeypatch, plan, 1), _compile(monkeypatch, plan, 0)
+    args = _dev(b.p_values, b.a_values, b.q, b.l, b.u)
+    for warm in (None, tuple(_dev(*_warm(plan, batch, 8)))):
+        got = band.engine.solve(*args, warm=warm, check_termination=5)
+        assert native.stream_last_launch()["form"] == "band"
+        want = plain.engine.solve(*args, warm=warm, check_termination=5)
+        assert native.stream_last_launch()["form"] != "band"
+        for g, w in zip(got, want):
+            np.testing.assert_array_equal(g.cpu().numpy(), w.cpu().numpy())
+        iters = band.engine.last_iters.cpu().numpy()
+        np.testing.assert_array_equal(iters, plain.engine.last_iters.cpu().numpy())
+        np.testing.assert_array_equal(band.engine.last_status.cpu().numpy(), plain.engine.last_status.cpu().numpy())
+
+
+@pytest.mark.parametrize("cls,batch", [(problems.SMALL, 75), (problems.CARTPOLE, 5000)],
+                         ids=lambda v: getattr(v, "name", str(v)))
+def test_band_form_adaptive_rho(cuda_device, monkeypatch, cls, batch):
+    b = problems.make_batch(cls, batch, seed=37)
+    settings = OSQPSettings(**{**problems.DEFAULT_SETTINGS, "max_iter": 30, "adaptive_rho": True,
+                               "adaptive_rho_interval": 8, "adaptive_rho_tolerance": 2.0})
+    plan = problems.make_plan(b, settings)
+    band, plain = _compile(monkeypatch, plan, 1), _compile(monkeypatch, plan, 0)
+    args = _dev(b.p_values, b.a_values, b.q, b.l, b.u)
+    got, want = band.engine.solve(*args), plain.engine.solve(*args)
+    for g, w in zip(got, want):
+        np.testing.assert_array_equal(g.cpu().numpy(), w.cpu().numpy())
+    upd = band.engine.last_rho_updates.cpu().numpy()
+    np.testing.assert_array_equal(upd, plain.engine.last_rho_updates.cpu().numpy())
+    assert upd.sum() > 0
+
+
+@pytest.mark.parametrize("check", [0, 5])
+def test_band_form_classes(cuda_device, monkeypatch, check):
+    """Classes of both window widths in one launch, several tiles per CTA."""
+    specs = [(problems.QUADROTOR, 2000), (problems.SMALL, 3001), (problems.CARTPOLE, 1500)]
+    items = {0: [], 1: []}
+    for k, (cls, batch) in enumerate(specs):
+        b = problems.make_batch(cls, batch, seed=20 + k)
+        plan = problems.make_plan(b, OSQPSettings(**{**problems.DEFAULT_SETTINGS, "max_iter": 30}))
+        for f in (0, 1):
+            items[f].append((_compile(monkeypatch, plan, f).engine, *_dev(b.p_values, b.a_values, b.q, b.l, b.u), None))
+    got = solve_classes(items[1], check_termination=check)
+    assert native.stream_last_launch()["form"] == "band"
+    want = solve_classes(items[0], check_termination=check)
+    for gs, ws in zip(got, want):
+        for g, w in zip(gs, ws):
+            np.testing.assert_array_equal(g.cpu().numpy(), w.cpu().numpy())
+
+
+def test_band_form_choice(cuda_device):
+    """Which form a solve runs by default: long chains the band form, others
+    the streaming forms where one tile per SM does not bound them."""
+    for cls, batch, band in ((problems.QUADROTOR, 40, True), (problems.CARTPOLE, 5000, True), (problems.SMALL, 40, False)):
+        b = problems.make_batch(cls, batch, seed=1)
+        comp = compile_osqp(problems.make_plan(b), np.float32, qdldl_backend="cuda", transpose_work=True)
+        comp.engine.solve(*_dev(b.p_values, b.a_values, b.q, b.l, b.u))
+        assert (native.stream_last_launch()["form"] == "band") == band, cls.name
+
+
+def test_band_form_wait_timeout(cuda_device, monkeypatch):
+    """Waits limited to one microsecond give up: every instance is marked, the
+    launch returns, and the next solve is right."""
+    import torch
+
+    b = problems.make_batch(problems.CARTPOLE, 96, seed=5)
+    plan = problems.make_plan(b)
+    comp = _compile(monkeypatch, plan, 1)
+    args = _dev(b.p_values, b.a_values, b.q, b.l, b.u)
+    monkeypatch.setenv("WMPC_STREAM_WAIT_LIMIT_NS", "1000")
+    comp.engine.solve(*args)
+    torch.cuda.synchronize()
+    assert native.stream_last_launch()["form"] == "band"
+    status = comp.engine.last_status.cpu().numpy()
+    assert np.all(status & native.STATUS_KERNEL_ABORT), np.unique(status)
+    monkeypatch.delenv("WMPC_STREAM_WAIT_LIMIT_NS")
+    got = comp.engine.solve(*args)
+    assert not np.any(comp.engine.last_status.cpu().numpy() & native.STATUS_KERNEL_ABORT)
+    ref = osqp_ref.solve(plan, b.p_values, b.a_values, b.q, b.l, b.u)
+    for g, r in zip(got[:3], ref[:3]):
+        np.testing.assert_array_equal(g.cpu().numpy(), r)

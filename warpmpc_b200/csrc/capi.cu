@@ -2,12 +2,14 @@
 // include/warpmpc_b200.h).  Argument validation, table upload, error
 // reporting; all numerics live in qdldl.cu / osqp.cu.
 #include <atomic>
+#include <climits>
 #include <cstring>
 #include <mutex>
 #include <numeric>
 #include <string>
 #include <vector>
 
+#include "band.cuh"
 #include "common.cuh"
 #include "osqp.cuh"
 #include "qdldl.cuh"
@@ -269,6 +271,113 @@ bool build_stream_plan(const HostPattern& hp, const StreamTargets& targets, cons
   *out = sp;
   return true;
 }
+
+// The band form of an OSQP problem: its tables, and the factorization tables
+// that write its stream.  False (why set) where the pattern has none.
+bool build_band_plan(const HostPattern& hp, const wmpc_osqp_desc* desc, const std::vector<float>& unscale,
+                     BandPlan* out, StreamPlan* factor, void** block, std::string* why) {
+  HostBand hb;
+  std::vector<int> init_slot, upd_ptr;
+  std::vector<unsigned short> upd_slot16;
+  int max_row = 0;
+  if (!build_band_tables(hp, desc->rho_vec, desc->rho_inv_vec, desc->rho_type, desc->n, unscale.data(), &hb, why) ||
+      !build_factor_tables(hp, &init_slot, &upd_ptr, &upd_slot16, &max_row, why))
+    return false;
+  BandPlan bp{};
+  bp.n = hb.n;
+  bp.n_prim = hb.n_prim;
+  bp.n_pre = hb.n_pre;
+  bp.T = hb.T;
+  bp.T4 = hb.T4;
+  bp.units = hb.units;
+  bp.n_chunks = hb.n_chunks;
+  bp.chunk_cols = hb.chunk_cols;
+  bp.n_yr = hb.n_yr;
+  bp.nb = hb.nb;
+  bp.blen = hb.blen;
+  bp.chunk_bytes = hb.chunk_bytes;
+  bp.item_bytes = hb.item_bytes;
+  bp.n_rows = static_cast<int>(hb.rec_off.size());
+  StreamPlan sp{};
+  sp.n = hp.n;
+  sp.nnz_l = hp.nnz_l;
+  sp.blen = sp.flen = hb.blen;
+  sp.max_row_nnz = max_row;
+  sp.n_pad_b = static_cast<int>(hb.pad.size());
+  std::vector<int> upd_slot(upd_slot16.begin(), upd_slot16.end());
+  std::vector<int> row_info, upd_pos, step_doff(hp.nnz_l), boff(hp.nnz_l), foff(hp.nnz_l);
+  for (int k = 0; k < hp.n; ++k) {
+    const int p0 = hp.proc_ptr[k], p1 = hp.proc_ptr[k + 1], i0 = hp.init_ptr[k], i1 = hp.init_ptr[k + 1];
+    sp.max_row_kv = std::max(sp.max_row_kv, 1 + i1 - i0);
+    row_info.insert(row_info.end(), {p0, p1, i0, i1, upd_ptr[p0], upd_ptr[p1], hb.dpos[k], k + i0});
+    for (int e = p0; e < p1; ++e) {
+      const int c = hp.proc_cols[e];
+      step_doff[e] = hb.dpos[c];
+      boff[e] = hb.lpos[hp.proc_lidx[e]];
+      foff[e] = hb.lpos2[hp.proc_lidx[e]];
+      for (int q = 0; q < hp.proc_offsets[e]; ++q) upd_pos.push_back(hb.lpos[hp.lp[c] + q]);
+    }
+  }
+  Packer sk;
+  sk.add(hb.col_word.data(), hb.col_word.size(), &bp.col_word);
+  sk.add(hb.chunk.data(), hb.chunk.size(), reinterpret_cast<const int**>(&bp.chunk));
+  sk.add(hb.far_ptr.data(), hb.far_ptr.size(), &bp.far_ptr);
+  sk.add(hb.far.data(), hb.far.size(), reinterpret_cast<const int**>(&bp.far));
+  sk.add(hb.item.data(), hb.item.size(), &bp.item);
+  sk.add(hb.rec.data(), hb.rec.size(), &bp.rec);
+  sk.add(hb.rec_off.data(), hb.rec_off.size(), &bp.rec_off);
+  sk.add(hb.iter_off.data(), hb.iter_off.size(), &bp.iter_off);
+  sk.add(hb.param_off.data(), hb.param_off.size(), &bp.param_off);
+  sk.add(row_info.data(), row_info.size(), reinterpret_cast<const int**>(&sp.row_info));
+  sk.add(init_slot.data(), init_slot.size(), &sp.init_slot);
+  sk.add(upd_ptr.data(), upd_ptr.size(), &sp.upd_ptr);
+  sk.add(upd_slot.data(), upd_slot.size(), &sp.upd_slot);
+  sk.add(upd_pos.data(), upd_pos.size(), &sp.upd_pos);
+  sk.add(step_doff.data(), step_doff.size(), &sp.step_doff);
+  sk.add(boff.data(), boff.size(), &sp.proc_boff);
+  sk.add(foff.data(), foff.size(), &sp.proc_foff);
+  sk.add(hb.pad.data(), hb.pad.size(), &sp.pad_boff);
+  int* sblock = nullptr;
+  if (sk.upload(&sblock) != WMPC_OK) {
+    *why = g_last_error;
+    return false;
+  }
+  *block = sblock;
+  *out = bp;
+  *factor = sp;
+  return true;
+}
+
+// Schedule knobs in the environment ask for the unit schedules of the
+// streaming form; WMPC_STREAM_BAND=0 / 1 turns the band form off / on.
+bool band_wanted() {
+  if (const char* v = getenv("WMPC_STREAM_BAND")) return atoi(v) != 0;
+  for (const char* k : {"WMPC_STREAM_UNITS", "WMPC_STREAM_COLS", "WMPC_STREAM_REL", "WMPC_STREAM_FUNITS",
+                        "WMPC_STREAM_OFFLOAD", "WMPC_STREAM_LSTAGES", "WMPC_STREAM_SSTAGES",
+                        "WMPC_STREAM_FRONTIER_LAG", "WMPC_STREAM_FRONTIER_COPIES"})
+    if (getenv(k)) return false;
+  const char* f = getenv("WMPC_STREAM_FRONTIER");
+  return !f || atoi(f) == 2;
+}
+
+// Tiles (of 32 instances) up to which a solve runs the band form.  Its fixed
+// cost is the pre-chain, whose columns and rows one warp does before the others
+// may go on (some 2.5 us per column and iteration, against 0.2 per chain row):
+// it loses where the chain is not much longer.  Where the chain is 10 to 20
+// times as long it wins only up to one tile per SM: with more, the streaming
+// form shares an SM between two or three tiles.  ADMM of 25 iterations, us, band
+// against streaming form, at 2000 / 9000 / 60,000 instances:
+//   20-step 6-state class (T 79, 12)     1059 / 1599 / 10408 against  937 / 1135 / 8172
+//   10-step quadrotor class (T 121, 7)   1323 / 2671 / 17380 against 1800 / 2401 / 16562
+//   40-step 6-state class (T 159, 12)    1555 / 3109 / 20639 against 1830 / 2597 / 17764
+//   20-step cartpole class (T 83, 4)      618 / 1062 /  6908 against  898 / 1059 / 8041
+//   20-step quadrotor class (T 241, 7)   2064 / 4160 / 26825 against 3506 / 5056 / 35956
+int band_tile_limit(const BandPlan& bp, int num_sms) {
+  if (getenv("WMPC_STREAM_BAND")) return INT_MAX;  // asked for
+  if (bp.T >= 20 * bp.n_pre) return INT_MAX;
+  return bp.T >= 10 * bp.n_pre ? num_sms : 0;
+}
+
 }  // namespace
 }  // namespace wmpc
 
@@ -400,6 +509,37 @@ int wmpc_stream_schedule_host(const wmpc_pattern_desc* desc, const float* rho, c
   app(hs.pad_boff); app(hs.pad_foff);
   app(hs.chunk_pre_u0); app(hs.chunk_pre_units);
   w.push_back(hs.frontier_slots); w.push_back(hs.frontier_lag); w.push_back(hs.max_frows);
+  *out_words = static_cast<int64_t>(w.size());
+  if (!out) return WMPC_OK;
+  if (out_capacity < static_cast<int64_t>(w.size())) return fail(WMPC_ERR_INVALID_ARGUMENT, "output buffer too small");
+  std::memcpy(out, w.data(), w.size() * sizeof(int32_t));
+  return WMPC_OK;
+}
+
+int wmpc_band_tables_host(const wmpc_pattern_desc* desc, const float* rho, const float* rhoinv, int32_t n_primal,
+                          int32_t* out, int64_t out_capacity, int64_t* out_words) {
+  if (!desc || !out_words || !rho || !rhoinv) return fail(WMPC_ERR_INVALID_ARGUMENT, "null argument");
+  const int n = desc->n, nnz_l = desc->nnz_l;
+  if (n <= 0 || nnz_l < 0 || n_primal < 0 || n_primal > n) return fail(WMPC_ERR_INVALID_ARGUMENT, "bad sizes");
+  HostPattern hp;
+  hp.n = n;
+  hp.nnz_a = desc->nnz_a;
+  hp.nnz_l = nnz_l;
+  hp.lp.assign(desc->lp, desc->lp + n + 1);
+  hp.li.assign(desc->li, desc->li + nnz_l);
+  hp.p.assign(desc->p, desc->p + n);
+  std::string why;
+  HostBand hb;
+  if (!build_band_tables(hp, rho, rhoinv, nullptr, n_primal, nullptr, &hb, &why))
+    return fail(WMPC_ERR_UNSUPPORTED, "%s", why.c_str());
+  std::vector<int> w{hb.n, hb.n_prim, hb.n_pre, hb.T, hb.T4, hb.units, hb.n_chunks, hb.chunk_cols, hb.n_yr, hb.nb,
+                     hb.blen, hb.chunk_bytes, hb.item_bytes,
+                     (int)hb.far.size(), (int)hb.rec_off.size(), (int)hb.pad.size()};
+  auto app = [&](const std::vector<int>& v, size_t count) { w.insert(w.end(), v.begin(), v.begin() + count); };
+  app(hb.col_word, hb.T4); app(hb.chunk, hb.chunk.size()); app(hb.far_ptr, hb.n_chunks); app(hb.far, hb.far.size());
+  app(hb.item, hb.item.size()); app(hb.rec, hb.rec.size()); app(hb.rec_off, hb.rec_off.size());
+  app(hb.iter_off, n); app(hb.param_off, n); app(hb.lpos, nnz_l); app(hb.lpos2, nnz_l); app(hb.dpos, n);
+  app(hb.pad, hb.pad.size());
   *out_words = static_cast<int64_t>(w.size());
   if (!out) return WMPC_OK;
   if (out_capacity < static_cast<int64_t>(w.size())) return fail(WMPC_ERR_INVALID_ARGUMENT, "output buffer too small");
@@ -850,6 +990,10 @@ int wmpc_osqp_create(const wmpc_osqp_desc* desc, const wmpc_plan* kkt_plan, wmpc
                          stream_max_ctas(q->spf, kkt_plan->device, q->ctas_limit) >
                              stream_max_ctas(q->sp, kkt_plan->device, q->ctas_limit);
     }
+    std::string why;
+    q->has_band = q->has_stream && band_wanted() &&
+                  build_band_plan(hp, desc, unscale, &q->bp, &q->band_factor, &q->band_block, &why);
+    if (q->has_band) q->band_tiles = band_tile_limit(q->bp, q->num_sms);
   }
   *out = q;
   return WMPC_OK;
@@ -861,6 +1005,7 @@ int wmpc_osqp_destroy(wmpc_osqp* osqp) {
   if (osqp->block) cudaFree(osqp->block);
   if (osqp->stream_block) cudaFree(osqp->stream_block);
   if (osqp->stream_block_f) cudaFree(osqp->stream_block_f);
+  if (osqp->band_block) cudaFree(osqp->band_block);
   delete osqp;
   return WMPC_OK;
 }

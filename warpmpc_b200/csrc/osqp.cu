@@ -7,6 +7,7 @@
 // residuals 866-871); -fmad=false keeps every product and sum separately
 // rounded.
 #include "common.cuh"
+#include <algorithm>
 #include <vector>
 
 #include "osqp.cuh"
@@ -633,9 +634,10 @@ Layout carve(const Osqp& o, const Pattern& pat, int batch, int pb, int ab, int m
     L.x = c.take((size_t)o.n * batch);
     L.z = c.take((size_t)o.m * batch);
     L.y = c.take((size_t)o.m * batch);
-    // (either schedule a launch may pick)
-    L.stream_ws = c.take(std::max(stream_workspace_floats(q->sp, batch),
-                                  q->has_frontier ? stream_workspace_floats(q->spf, batch) : (size_t)0));
+    // (whichever schedule a launch may pick)
+    L.stream_ws = c.take(std::max({stream_workspace_floats(q->sp, batch),
+                                   q->has_frontier ? stream_workspace_floats(q->spf, batch) : (size_t)0,
+                                   q->has_band ? band_workspace_floats(q->bp, batch) : (size_t)0}));
     L.stream_status = reinterpret_cast<int*>(c.take((size_t)((batch + 31) / 32) * 32));
     L.error_word = reinterpret_cast<int*>(c.take(4));
     if (o.rho_type) {  // per-instance rho (adaptation)
@@ -707,6 +709,9 @@ int stream_begin(const Pattern& pat, const StreamPlan& sp, const Osqp& o, const 
                  const float* qs, const float* ls, const float* us, bool warm, bool track, float* work,
                  int* status, int batch, int num_sms, bool reuse_factor, StreamJobDesc* job, cudaStream_t s,
                  const float* rinv_rows = nullptr, const int* only = nullptr);
+int stream_factor(const Pattern& pat, const StreamPlan& sp, const Osqp& o, const float* pT, long long ldp, int sbp,
+                  const float* aT, long long lda, int sba, float* bstream, float* fstream, int* status, int batch,
+                  int num_sms, cudaStream_t s, const float* rinv_rows = nullptr, const int* only = nullptr);
 int stream_run(const StreamJobDesc* jobs, int n_jobs, int* error, int num_sms, cudaStream_t s);
 int stream_end(const StreamPlan& sp, const Osqp& o, const StreamJobDesc& job, float* x, float* z, float* y,
                cudaStream_t s);
@@ -831,6 +836,49 @@ int stream_solve_begin(const wmpc_osqp& q, const wmpc_osqp_options& opt, const w
   return WMPC_OK;
 }
 
+bool band_for(const wmpc_osqp& q, int tiles) { return q.has_band && tiles <= q.band_tiles; }
+
+// The band form's first half: inputs staged, factor, state records; fills `job`.
+int band_prepare(const wmpc_osqp& q, const wmpc_osqp_options& opt, const wmpc_osqp_batch& d, const Layout& L,
+                 bool warm, bool reuse_factor, BandJobDesc* job, cudaStream_t s, const float* rinv_rows = nullptr,
+                 const int* only = nullptr) {
+  const Osqp& o = q.dev;
+  const int B = d.batch, pb = d.p_batch, ab = d.a_batch;
+  const int check = opt.check_termination > 0 ? opt.check_termination : 0;
+  const BandWork w = band_work(q.bp, B, L.stream_ws);
+  int rc;
+  if (!reuse_factor &&
+      (rc = stream_factor(q.kkt_plan->pat, q.band_factor, o, L.pT, pb, pb > 1 ? 1 : 0, L.aT, ab, ab > 1 ? 1 : 0,
+                          w.stream, w.stream, L.stream_status, B, q.num_sms, s, rinv_rows, only)))
+    return rc;
+  if ((rc = band_state_in(q.bp, o, L.aT, ab, ab > 1 ? 1 : 0, check > 0, warm, L.x, L.z, L.y, L.qs, L.ls, L.us, w, B,
+                          s)))
+    return rc;
+  *job = BandJobDesc{};
+  job->bp = q.bp;
+  job->stream = w.stream;
+  job->pres = w.pres;
+  job->n_tiles = w.tiles;
+  job->batch = B;
+  job->max_iter = opt.max_iter;
+  job->check_every = check;
+  job->ctas_limit = q.ctas_limit;
+  job->chg_eps = opt.eps_abs;
+  job->iters = check ? d.iters : nullptr;
+  job->sigma = o.sigma;
+  job->alpha = o.alpha;
+  job->one_minus_alpha = o.one_minus_alpha;
+  return WMPC_OK;
+}
+
+int band_solve_begin(const wmpc_osqp& q, const wmpc_osqp_options& opt, const wmpc_osqp_batch& d, const Layout& L,
+                     BandJobDesc* job, cudaStream_t s) {
+  int rc;
+  if ((rc = stage_inputs(q.dev, opt, d, L, s))) return rc;
+  WMPC_CUDA_TRY(cudaMemsetAsync(L.error_word, 0, sizeof(int), s));
+  return band_prepare(q, opt, d, L, opt.warm_start != 0, opt.reuse_factor != 0, job, s);
+}
+
 // Streaming solve with per-instance rho adaptation (fixed iterations): the
 // iterations run in launches of adaptive_rho_interval; between two, the state
 // comes back, each instance estimates its rho (rho_update_kernel, the plain
@@ -853,7 +901,17 @@ int stream_solve_adaptive(const wmpc_osqp& q, const wmpc_osqp_options& opt, cons
   rho_init_kernel<<<rgrid, 128, 0, s>>>(o, L.rho_row, L.rinv_row, L.rho_b, L.rho_count, B);
   WMPC_LAUNCH_CHECK();
   State st{L.x, L.z, L.y, L.qs, L.ls, L.us, B};
+  BandJobDesc band;
+  const bool use_band = band_for(q, (B + 31) / 32);
   auto begin = [&](bool warm, const int* only) -> int {
+    if (use_band) {
+      const int r = band_prepare(q, opt, d, L, warm, false, &band, s, L.rinv_row, only);
+      band.check_every = 0;
+      band.iters = nullptr;
+      band.rho_b = L.rho_b;
+      band.rho_count = L.rho_count;
+      return r;
+    }
     int r = stream_begin(q.kkt_plan->pat, sp, o, L.pT, pb, sbp, L.aT, ab, sba, L.x, L.z, L.y, L.qs, L.ls, L.us, warm,
                          false, L.stream_ws, L.stream_status, B, q.num_sms, false, job, s, L.rinv_row, only);
     job->check_every = 0;
@@ -868,11 +926,15 @@ int stream_solve_adaptive(const wmpc_osqp& q, const wmpc_osqp_options& opt, cons
   const int interval = opt.adaptive_rho_interval;
   for (int it = 0; it < opt.max_iter;) {
     const int seg = opt.max_iter - it < interval ? opt.max_iter - it : interval;
-    job->max_iter = seg;
-    if ((rc = stream_run(job, 1, L.error_word, q.num_sms, s))) return rc;
+    job->max_iter = band.max_iter = seg;
+    if ((rc = use_band ? band_run(&band, 1, L.error_word, q.num_sms, s)
+                       : stream_run(job, 1, L.error_word, q.num_sms, s)))
+      return rc;
     it += seg;
     if (it < opt.max_iter) {
-      if ((rc = stream_end(sp, o, *job, L.x, L.z, L.y, s))) return rc;
+      if ((rc = use_band ? band_state_out(q.bp, band_work(q.bp, B, L.stream_ws), L.x, L.z, L.y, B, s)
+                         : stream_end(sp, o, *job, L.x, L.z, L.y, s)))
+        return rc;
       rho_update_kernel<<<ceil_div(B, 128), 128, 0, s>>>(o, L.pT, pb, sbp, L.aT, ab, sba, st, L.rho_row, L.rinv_row,
                                                          L.rho_b, L.rho_changed, L.rho_count,
                                                          opt.adaptive_rho_tolerance, B);
@@ -888,13 +950,16 @@ int stream_solve_adaptive(const wmpc_osqp& q, const wmpc_osqp_options& opt, cons
 }
 
 // Streaming solve, second half: state back, exact residuals and status, outputs.
+// (job null: the band form's state)
 int stream_solve_end(const wmpc_osqp& q, const wmpc_osqp_options& opt, const wmpc_osqp_batch& d, const Layout& L,
-                     const StreamJobDesc& job, const int* error_word, cudaStream_t s) {
+                     const StreamJobDesc* job, const int* error_word, cudaStream_t s) {
   const Osqp& o = q.dev;
   const int B = d.batch, pb = d.p_batch, ab = d.a_batch;
   const int check = opt.check_termination > 0 ? opt.check_termination : 0;
   int rc;
-  if ((rc = stream_end(job.sp, o, job, L.x, L.z, L.y, s))) return rc;
+  if ((rc = job ? stream_end(job->sp, o, *job, L.x, L.z, L.y, s)
+                : band_state_out(q.bp, band_work(q.bp, B, L.stream_ws), L.x, L.z, L.y, B, s)))
+    return rc;
   State st{L.x, L.z, L.y, L.qs, L.ls, L.us, B};
   if (residuals_wanted(opt, d)) {
     residual_kernel<<<ceil_div(B, 32), dim3(32, kResParts), 0, s>>>(
@@ -949,14 +1014,20 @@ int osqp_solve(const wmpc_osqp& q, const wmpc_osqp_options& opt, const wmpc_osqp
   if (L.streaming && adaptive) {
     StreamJobDesc job;
     if ((rc = stream_solve_adaptive(q, opt, d, L, &job, s))) return rc;
-    return stream_solve_end(q, opt, d, L, job, L.error_word, s);
+    return stream_solve_end(q, opt, d, L, band_for(q, (B + 31) / 32) ? nullptr : &job, L.error_word, s);
+  }
+  if (L.streaming && band_for(q, (B + 31) / 32)) {
+    BandJobDesc job;
+    if ((rc = band_solve_begin(q, opt, d, L, &job, s))) return rc;
+    if ((rc = band_run(&job, 1, L.error_word, q.num_sms, s))) return rc;
+    return stream_solve_end(q, opt, d, L, nullptr, L.error_word, s);
   }
   if (L.streaming) {
     StreamJobDesc job;
     const bool frontier = frontier_for(q, opt.check_termination > 0, (B + 31) / 32);
     if ((rc = stream_solve_begin(q, opt, d, L, frontier, &job, s))) return rc;
     if ((rc = stream_run(&job, 1, L.error_word, q.num_sms, s))) return rc;
-    return stream_solve_end(q, opt, d, L, job, L.error_word, s);
+    return stream_solve_end(q, opt, d, L, &job, L.error_word, s);
   }
   if ((rc = stage_inputs(o, opt, d, L, s))) return rc;
   State st{L.x, L.z, L.y, L.qs, L.ls, L.us, B};
@@ -1090,15 +1161,27 @@ int osqp_solve_multi(const wmpc_osqp* const* qs, const wmpc_osqp_options* opts, 
   if (n < 1 || n > 6) return fail(WMPC_ERR_INVALID_ARGUMENT, "1 to 6 classes per launch, got %d", n);
   std::vector<Layout> L(n);
   std::vector<StreamJobDesc> jobs(n);
+  std::vector<BandJobDesc> band_jobs(n);
   std::vector<int> active;
   int rc;
-  // one schedule form per launch: the frontier form only when every class
-  // would pick it for the launch's tiles
-  bool frontier = true;
+  // one schedule form per launch: the band form where the classes that would
+  // pick it for the launch's tiles hold most of its work (and all of them have
+  // it and fit), else the frontier form only when every class would pick it
+  bool frontier = true, band = true;
   int tiles = 0;
+  double all_work = 0.0, band_work_part = 0.0;
+  std::vector<const BandPlan*> plans;
   for (int i = 0; i < n; ++i) tiles += ds[i].batch > 0 ? (ds[i].batch + 31) / 32 : 0;
   for (int i = 0; i < n; ++i)
-    if (ds[i].batch > 0) frontier = frontier && frontier_for(*qs[i], opts[i].check_termination > 0, tiles);
+    if (ds[i].batch > 0) {
+      const double work = (double)((ds[i].batch + 31) / 32) * qs[i]->kkt_plan->pat.nnz_l;
+      all_work += work;
+      if (band_for(*qs[i], tiles)) band_work_part += work;
+      band = band && qs[i]->has_band;
+      plans.push_back(&qs[i]->bp);
+      frontier = frontier && frontier_for(*qs[i], opts[i].check_termination > 0, tiles);
+    }
+  band = band && 2.0 * band_work_part >= all_work && band_fits(plans.data(), (int)plans.size());
   for (int i = 0; i < n; ++i) {
     const wmpc_osqp& q = *qs[i];
     const wmpc_osqp_batch& d = ds[i];
@@ -1112,16 +1195,25 @@ int osqp_solve_multi(const wmpc_osqp* const* qs, const wmpc_osqp_options* opts, 
                  static_cast<char*>(ws[i]), &need, &q, true);
     if (ws[i] == nullptr || ws_bytes[i] < need)
       return fail(WMPC_ERR_WORKSPACE, "class %d needs %zu workspace bytes, got %zu", i, need, ws_bytes[i]);
-    if ((rc = stream_solve_begin(q, opts[i], d, L[i], frontier, &jobs[i], s))) return rc;
+    if ((rc = band ? band_solve_begin(q, opts[i], d, L[i], &band_jobs[i], s)
+                   : stream_solve_begin(q, opts[i], d, L[i], frontier, &jobs[i], s)))
+      return rc;
     active.push_back(i);
   }
   if (active.empty()) return WMPC_OK;
   std::vector<StreamJobDesc> run;
-  for (int i : active) run.push_back(jobs[i]);
+  std::vector<BandJobDesc> band_run_jobs;
+  for (int i : active) {
+    run.push_back(jobs[i]);
+    band_run_jobs.push_back(band_jobs[i]);
+  }
   int* error_word = L[active[0]].error_word;
-  if ((rc = stream_run(run.data(), static_cast<int>(run.size()), error_word, qs[active[0]]->num_sms, s))) return rc;
+  const int n_run = static_cast<int>(active.size()), sms = qs[active[0]]->num_sms;
+  if ((rc = band ? band_run(band_run_jobs.data(), n_run, error_word, sms, s)
+                 : stream_run(run.data(), n_run, error_word, sms, s)))
+    return rc;
   for (int i : active)
-    if ((rc = stream_solve_end(*qs[i], opts[i], ds[i], L[i], jobs[i], error_word, s))) return rc;
+    if ((rc = stream_solve_end(*qs[i], opts[i], ds[i], L[i], band ? nullptr : &jobs[i], error_word, s))) return rc;
   return WMPC_OK;
 }
 

@@ -1,6 +1,7 @@
 // Device-side OSQP problem description (one FixedOSQPPlan) and launchers.
 #pragma once
 
+#include "band.cuh"
 #include "common.cuh"
 #include "stream.cuh"
 
@@ -67,5 +68,11 @@ struct wmpc_osqp {
   bool frontier_pays = false;  // it fits two CTAs per SM where sp does not
   wmpc::StreamPlan spf{};
   void* stream_block_f = nullptr;
+  // the band form (band.cuh): run by persistent solves of at most band_tiles tiles
+  bool has_band = false;
+  int band_tiles = 0;
+  wmpc::BandPlan bp{};
+  wmpc::StreamPlan band_factor{};  // the factorization's tables, writing the band form's stream
+  void* band_block = nullptr;
   std::string stream_why;  // why the streaming path is unavailable (diagnostics)
 };

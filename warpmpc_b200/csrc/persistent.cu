@@ -1533,6 +1533,39 @@ size_t stream_workspace_floats(const StreamPlan& sp, int batch) {
   return tiles * ((size_t)sp.blen + (size_t)sp.flen + vectors * 32 * (size_t)sp.n) + 64;
 }
 
+// Factorization of a batch into a schedule's streams (rinv_rows: per-instance
+// 1/rho inputs; only: just the tiles holding a marked instance).
+int stream_factor(const Pattern& pat, const StreamPlan& sp, const Osqp& o, const float* pT, long long ldp, int sbp,
+                  const float* aT, long long lda, int sba, float* bstream, float* fstream, int* status, int batch,
+                  int num_sms, cudaStream_t s, const float* rinv_rows, const int* only) {
+  const int n_tiles = (batch + 31) / 32;
+  OsqpInputs in{pT, ldp, sbp, aT, lda, sba, rinv_rows, rinv_rows ? (long long)batch : 0};
+  if (rinv_rows && !o.kin_desc_rho) return fail(WMPC_ERR_UNSUPPORTED, "the problem has no per-instance rho inputs");
+  // L-batch sized so that every tile's warp is resident at once (all of a
+  // launch's rows then wait out their round trips together)
+  const int warps = 2;
+  const int per_sm = ceil_div(n_tiles, num_sms > 0 ? num_sms : 1);
+  const int budget_floats = (200 * 1024 / 4) / (per_sm > 0 ? per_sm : 1);
+  int lbatch = (budget_floats - factor_warp_words(sp, 0)) / 33;
+  // WMPC_FACTOR_LBATCH fixes the batch instead (tuning: fewer resident
+  // warps, fewer round trips per row)
+  // with many tiles per SM a short batch measured faster (16: 8.98 ms against 9.23 for the budget's
+  // 24 on 65,536 quadrotor instances; 32 to 128: 11.9 to 16.5 ms): the smaller shared-memory
+  // request leaves more of the SM's unified memory to L1, which serves the index tables
+  if (per_sm >= 8 && lbatch > 16) lbatch = 16;
+  if (const char* v = getenv("WMPC_FACTOR_LBATCH")) lbatch = atoi(v);
+  lbatch = lbatch < 8 ? 8 : (lbatch > 128 ? 128 : lbatch);
+  const size_t smem = (size_t)warps * factor_warp_words(sp, lbatch) * sizeof(float);
+  if (smem > (size_t)kMaxSmemBytes) return fail(WMPC_ERR_UNSUPPORTED, "factor rows too long for shared memory");
+  WMPC_CUDA_TRY(cudaFuncSetAttribute(factor_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  profile_mark_begin(s, kProfileFactor);
+  factor_stream_kernel<<<ceil_div(n_tiles, warps), warps * 32, smem, s>>>(pat, sp, o, in, bstream, fstream, status,
+                                                                          n_tiles, batch, lbatch, only);
+  profile_mark_end(s, kProfileFactor);
+  WMPC_LAUNCH_CHECK();
+  return WMPC_OK;
+}
+
 // Factorization into the streams and the state into its records (one class).
 int stream_begin(const Pattern& pat, const StreamPlan& sp, const Osqp& o, const float* pT, long long ldp, int sbp,
                  const float* aT, long long lda, int sba, const float* x, const float* z, const float* y,
@@ -1553,30 +1586,10 @@ int stream_begin(const Pattern& pat, const StreamPlan& sp, const Osqp& o, const 
   float* rhs = sp.frontier_slots > 0 ? pres + tl * sp.n : nullptr;
   float* fwd = sp.frontier_slots > 0 ? rhs + tl * sp.n : nullptr;
   OsqpInputs in{pT, ldp, sbp, aT, lda, sba, rinv_rows, rinv_rows ? (long long)batch : 0};
-  if (rinv_rows && !o.kin_desc_rho) return fail(WMPC_ERR_UNSUPPORTED, "the problem has no per-instance rho inputs");
   if (!reuse_factor) {
-    // L-batch sized so that every tile's warp is resident at once (all of a
-    // launch's rows then wait out their round trips together)
-    const int warps = 2;
-    const int per_sm = ceil_div(n_tiles, num_sms > 0 ? num_sms : 1);
-    const int budget_floats = (200 * 1024 / 4) / (per_sm > 0 ? per_sm : 1);
-    int lbatch = (budget_floats - factor_warp_words(sp, 0)) / 33;
-    // WMPC_FACTOR_LBATCH fixes the batch instead (tuning: fewer resident
-    // warps, fewer round trips per row)
-    // with many tiles per SM a short batch measured faster (16: 8.98 ms against 9.23 for the budget's
-    // 24 on 65,536 quadrotor instances; 32 to 128: 11.9 to 16.5 ms): the smaller shared-memory
-    // request leaves more of the SM's unified memory to L1, which serves the index tables
-    if (per_sm >= 8 && lbatch > 16) lbatch = 16;
-    if (const char* v = getenv("WMPC_FACTOR_LBATCH")) lbatch = atoi(v);
-    lbatch = lbatch < 8 ? 8 : (lbatch > 128 ? 128 : lbatch);
-    const size_t smem = (size_t)warps * factor_warp_words(sp, lbatch) * sizeof(float);
-    if (smem > (size_t)kMaxSmemBytes) return fail(WMPC_ERR_UNSUPPORTED, "factor rows too long for shared memory");
-    WMPC_CUDA_TRY(cudaFuncSetAttribute(factor_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    profile_mark_begin(s, kProfileFactor);
-    factor_stream_kernel<<<ceil_div(n_tiles, warps), warps * 32, smem, s>>>(pat, sp, o, in, bstream, fstream, status,
-                                                                            n_tiles, batch, lbatch, only);
-    profile_mark_end(s, kProfileFactor);
-    WMPC_LAUNCH_CHECK();
+    const int rc = stream_factor(pat, sp, o, pT, ldp, sbp, aT, lda, sba, bstream, fstream, status, batch, num_sms, s,
+                                 rinv_rows, only);
+    if (rc) return rc;
   }
   {
     dim3 grid(ceil_div(tl, 128), sp.n < 1024 ? sp.n : 1024);

@@ -266,6 +266,11 @@ SIGNATURES = {
     "wmpc_quadrotor_jac_pattern": (ctypes.c_int, [_i32p, _i32p]),
     "wmpc_solve_tables_host": (ctypes.c_int, [ctypes.POINTER(PatternDesc), _i32p, ctypes.c_int64,
                                               ctypes.POINTER(ctypes.c_int64)]),
+    "wmpc_band_tables_host": (
+        ctypes.c_int,
+        [ctypes.POINTER(PatternDesc), _f32p, _f32p, ctypes.c_int32, _i32p, ctypes.c_int64,
+         ctypes.POINTER(ctypes.c_int64)],
+    ),
     "wmpc_stream_schedule_host": (
         ctypes.c_int,
         [ctypes.POINTER(PatternDesc), _f32p, _f32p, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
@@ -430,5 +435,5 @@ def stream_last_launch() -> dict:
     """The last streaming ADMM launch: schedule form, CTAs per SM, grid, shared memory."""
     info = (ctypes.c_int32 * 4)()
     check(lib().wmpc_stream_last_launch(info))
-    return {"form": {0: None, 1: "plain", 2: "frontier"}.get(int(info[0])), "ctas_per_sm": int(info[1]),
+    return {"form": {0: None, 1: "plain", 2: "frontier", 3: "band"}.get(int(info[0])), "ctas_per_sm": int(info[1]),
             "grid": int(info[2]), "smem_bytes": int(info[3])}

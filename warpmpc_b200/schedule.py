@@ -54,6 +54,36 @@ def solve_tables(qdldl_plan) -> dict:
     return {"tables": buf[2 : 2 + tw].copy(), "desc": buf[2 + tw : 2 + tw + 8 * n_chunks].reshape(n_chunks, 8).copy()}
 
 
+def band_tables(plan) -> dict | None:
+    """The band form's tables of an OSQP plan (``wmpc_band_tables_host``), or
+    None where its pattern has no such form."""
+    qp = plan.qdldl_plan
+    desc, keep, _ = _pattern_desc(qp)
+    lib = native.lib()
+    words = ctypes.c_int64()
+    rho, rinv = native.f32(plan.rho_vec), native.f32(plan.rho_inv_vec)
+    args = (ctypes.byref(desc), native.ptr_f32(rho), native.ptr_f32(rinv), int(plan.n))
+    rc = lib.wmpc_band_tables_host(*args, None, 0, ctypes.byref(words))
+    if rc == native.WMPC_ERR_UNSUPPORTED:
+        return None
+    native.check(rc)
+    buf = np.empty(words.value, dtype=np.int32)
+    native.check(lib.wmpc_band_tables_host(*args, native.ptr_i32(buf), buf.size, ctypes.byref(words)))
+    names = ("n", "n_prim", "n_pre", "T", "T4", "units", "n_chunks", "chunk_cols", "n_yr", "nb", "blen", "chunk_bytes",
+             "item_bytes", "n_far", "n_rows", "n_pad")
+    out = {k: int(v) for k, v in zip(names, buf)}
+    pos = len(names)
+    for name, count in (("col_word", out["T4"]), ("chunk", 4 * out["n_chunks"]), ("far_ptr", out["n_chunks"]),
+                        ("far", out["n_far"]), ("item", 2 * out["n_pre"] + out["nb"] + out["T"]),
+                        ("rec", 32 * out["n_rows"]), ("rec_off", out["n_rows"]), ("iter_off", qp.n),
+                        ("param_off", qp.n), ("lpos", qp.nnz_l), ("lpos2", qp.nnz_l), ("dpos", qp.n),
+                        ("pad", out["n_pad"])):
+        out[name] = buf[pos : pos + count].copy()
+        pos += count
+    assert pos == buf.size
+    return out
+
+
 def stream_schedule(plan, targets=DEFAULT_TARGETS) -> dict:
     """Schedule of an OSQP plan (rho per constraint) as NumPy arrays.
 
