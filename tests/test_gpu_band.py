@@ -156,3 +156,34 @@ def test_band_form_wait_timeout(cuda_device, monkeypatch):
     ref = osqp_ref.solve(plan, b.p_values, b.a_values, b.q, b.l, b.u)
     for g, r in zip(got[:3], ref[:3]):
         np.testing.assert_array_equal(g.cpu().numpy(), r)
+
+
+@pytest.mark.parametrize("band", [0, 1], ids=["stream", "band"])
+@pytest.mark.parametrize("cls,batch,shared", [(problems.SMALL, 37, True), (problems.CARTPOLE, 96, False),
+                                              (problems.SMALL, 1, False), (problems.QUADROTOR, 4801, True)],
+                         ids=lambda v: getattr(v, "name", str(v)))
+def test_given_factorization(cuda_device, monkeypatch, band, cls, batch, shared):
+    """A factorization given by the caller, shared or per instance: iterates
+    and status of the per-call kernels', a zero pivot reported for its instance."""
+    import torch
+
+    b = problems.make_batch(cls, batch, seed=12)
+    plan = problems.make_plan(b)
+    monkeypatch.setenv("WMPC_STREAM_FRONTIER", "2" if band else "0")
+    comp = _compile(monkeypatch, plan, band)
+    k = 1 if shared else batch
+    args = _dev(b.p_values[:k], b.a_values[:k], b.q, b.l, b.u)
+    lx, dinv = comp.factor(args[0], args[1])
+    if batch > 1 and not shared:
+        dinv[5, 17] = 0.0
+    warm = tuple(_dev(*_warm(plan, batch, 4)))
+    for w in (None, warm):
+        got = comp.engine.solve(*args, warm=w, factor=(lx, dinv))
+        assert native.stream_last_launch()["form"] == ("band" if band else "plain")
+        status = comp.engine.last_status.clone()
+        want = comp.engine.solve(*args, warm=w, factor=(lx, dinv), mode="plain")
+        for g, r in zip(got[:3], want[:3]):
+            assert torch.equal(g, r)
+        zero = (status & native.STATUS_ZERO_PIVOT) != 0
+        assert torch.equal(status & ~native.STATUS_ZERO_PIVOT, comp.engine.last_status)
+        assert zero.nonzero().flatten().tolist() == ([17] if batch > 1 and not shared else [])

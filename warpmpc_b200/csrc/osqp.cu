@@ -618,12 +618,26 @@ struct Layout {
   int* error_word;
 };
 
+constexpr size_t kMaxImportFloats = (size_t)12 << 30;  // 48 GiB
+
 // Workspace carve-up.  `external`: the caller supplies the factorization.
 Layout carve(const Osqp& o, const Pattern& pat, int batch, int pb, int ab, int mode, bool external, char* base,
              size_t* total, const wmpc_osqp* q = nullptr, bool use_stream = false, bool per_instance_factor = false) {
   Carve c{base};
   Layout L{};
-  if (use_stream && q && q->has_stream && mode == WMPC_OSQP_PERSISTENT && !external) {
+  // (either schedule a launch may pick)
+  const size_t stream_floats =
+      use_stream && q && q->has_stream
+          ? std::max({stream_workspace_floats(q->sp, batch),
+                      q->has_frontier ? stream_workspace_floats(q->spf, batch) : (size_t)0,
+                      q->has_band ? band_workspace_floats(q->bp, batch) : (size_t)0})
+          : 0;
+  // a given factorization is copied into the streams, one copy per instance: up
+  // to a bound (400,000 instances of the 30-step quadrotor class), past which the
+  // per-lane kernel reads it in place.  8192 instances of that class with one
+  // factorization, whole call: 6.75 ms streamed, 100.4 ms read in place.
+  if (use_stream && q && q->has_stream && mode == WMPC_OSQP_PERSISTENT &&
+      !(external && stream_floats > kMaxImportFloats)) {
     L.streaming = true;
     L.pT = c.take((size_t)o.nnz_p * pb);
     L.aT = c.take((size_t)o.nnz_a * ab);
@@ -634,10 +648,7 @@ Layout carve(const Osqp& o, const Pattern& pat, int batch, int pb, int ab, int m
     L.x = c.take((size_t)o.n * batch);
     L.z = c.take((size_t)o.m * batch);
     L.y = c.take((size_t)o.m * batch);
-    // (whichever schedule a launch may pick)
-    L.stream_ws = c.take(std::max({stream_workspace_floats(q->sp, batch),
-                                   q->has_frontier ? stream_workspace_floats(q->spf, batch) : (size_t)0,
-                                   q->has_band ? band_workspace_floats(q->bp, batch) : (size_t)0}));
+    L.stream_ws = c.take(stream_floats);
     L.stream_status = reinterpret_cast<int*>(c.take((size_t)((batch + 31) / 32) * 32));
     L.error_word = reinterpret_cast<int*>(c.take(4));
     if (o.rho_type) {  // per-instance rho (adaptation)
@@ -708,7 +719,9 @@ int stream_begin(const Pattern& pat, const StreamPlan& sp, const Osqp& o, const 
                  const float* aT, long long lda, int sba, const float* x, const float* z, const float* y,
                  const float* qs, const float* ls, const float* us, bool warm, bool track, float* work,
                  int* status, int batch, int num_sms, bool reuse_factor, StreamJobDesc* job, cudaStream_t s,
-                 const float* rinv_rows = nullptr, const int* only = nullptr);
+                 const float* rinv_rows = nullptr, const int* only = nullptr, const ExternalFactor* given = nullptr);
+int stream_import(const Pattern& pat, const StreamPlan& sp, const ExternalFactor& f, float* bstream, float* fstream,
+                  int* status, int batch, cudaStream_t s);
 int stream_factor(const Pattern& pat, const StreamPlan& sp, const Osqp& o, const float* pT, long long ldp, int sbp,
                   const float* aT, long long lda, int sba, float* bstream, float* fstream, int* status, int batch,
                   int num_sms, cudaStream_t s, const float* rinv_rows = nullptr, const int* only = nullptr);
@@ -810,7 +823,7 @@ static bool frontier_for(const wmpc_osqp& q, bool check, int tiles) {
 // Streaming solve, first half: inputs staged, factor, state records; fills
 // `job` (frontier: with the problem's frontier-form schedule).
 int stream_solve_begin(const wmpc_osqp& q, const wmpc_osqp_options& opt, const wmpc_osqp_batch& d, const Layout& L,
-                       bool frontier, StreamJobDesc* job, cudaStream_t s) {
+                       bool frontier, StreamJobDesc* job, cudaStream_t s, const ExternalFactor* given = nullptr) {
   const Osqp& o = q.dev;
   const int B = d.batch, pb = d.p_batch, ab = d.a_batch;
   const int check = opt.check_termination > 0 ? opt.check_termination : 0;
@@ -820,7 +833,7 @@ int stream_solve_begin(const wmpc_osqp& q, const wmpc_osqp_options& opt, const w
   if ((rc = stream_begin(q.kkt_plan->pat, frontier ? q.spf : q.sp, o, L.pT, pb, pb > 1 ? 1 : 0, L.aT, ab, ab > 1 ? 1 : 0,
                          L.x, L.z, L.y,
                          L.qs, L.ls, L.us, opt.warm_start != 0, check > 0, L.stream_ws, L.stream_status, B,
-                         q.num_sms, opt.reuse_factor != 0, job, s)))
+                         q.num_sms, opt.reuse_factor != 0, job, s, nullptr, nullptr, given)))
     return rc;
   // termination: an instance stops (freezes) once both its primal residual
   // (A x - z, carried exactly through the iterations) and its largest iterate
@@ -841,13 +854,16 @@ bool band_for(const wmpc_osqp& q, int tiles) { return q.has_band && tiles <= q.b
 // The band form's first half: inputs staged, factor, state records; fills `job`.
 int band_prepare(const wmpc_osqp& q, const wmpc_osqp_options& opt, const wmpc_osqp_batch& d, const Layout& L,
                  bool warm, bool reuse_factor, BandJobDesc* job, cudaStream_t s, const float* rinv_rows = nullptr,
-                 const int* only = nullptr) {
+                 const int* only = nullptr, const ExternalFactor* given = nullptr) {
   const Osqp& o = q.dev;
   const int B = d.batch, pb = d.p_batch, ab = d.a_batch;
   const int check = opt.check_termination > 0 ? opt.check_termination : 0;
   const BandWork w = band_work(q.bp, B, L.stream_ws);
   int rc;
-  if (!reuse_factor &&
+  if (given) {
+    if ((rc = stream_import(q.kkt_plan->pat, q.band_factor, *given, w.stream, w.stream, L.stream_status, B, s)))
+      return rc;
+  } else if (!reuse_factor &&
       (rc = stream_factor(q.kkt_plan->pat, q.band_factor, o, L.pT, pb, pb > 1 ? 1 : 0, L.aT, ab, ab > 1 ? 1 : 0,
                           w.stream, w.stream, L.stream_status, B, q.num_sms, s, rinv_rows, only)))
     return rc;
@@ -872,11 +888,11 @@ int band_prepare(const wmpc_osqp& q, const wmpc_osqp_options& opt, const wmpc_os
 }
 
 int band_solve_begin(const wmpc_osqp& q, const wmpc_osqp_options& opt, const wmpc_osqp_batch& d, const Layout& L,
-                     BandJobDesc* job, cudaStream_t s) {
+                     BandJobDesc* job, cudaStream_t s, const ExternalFactor* given = nullptr) {
   int rc;
   if ((rc = stage_inputs(q.dev, opt, d, L, s))) return rc;
   WMPC_CUDA_TRY(cudaMemsetAsync(L.error_word, 0, sizeof(int), s));
-  return band_prepare(q, opt, d, L, opt.warm_start != 0, opt.reuse_factor != 0, job, s);
+  return band_prepare(q, opt, d, L, opt.warm_start != 0, opt.reuse_factor != 0, job, s, nullptr, nullptr, given);
 }
 
 // Streaming solve with per-instance rho adaptation (fixed iterations): the
@@ -1006,8 +1022,14 @@ int osqp_solve(const wmpc_osqp& q, const wmpc_osqp_options& opt, const wmpc_osqp
       return fail(WMPC_ERR_INVALID_ARGUMENT, "adaptive_rho_tolerance must be at least 1");
   }
   size_t need = 0;
-  Layout L = carve(o, pat, B, pb, ab, mode, external, static_cast<char*>(ws), &need, &q, stream_eligible(q, &opt),
-                   adaptive);
+  if (external && fb_ext != 1 && fb_ext != B) return fail(WMPC_ERR_INVALID_ARGUMENT, "factor_batch must be 1 or batch");
+  // (the per-lane kernel's termination test is another one: it needs every iteration's residuals)
+  const bool use_stream = stream_eligible(q, &opt) && !(external && opt.check_termination > 0);
+  const ExternalFactor ext{lx_ext, dinv_ext, fb_ext};
+  const ExternalFactor* given = external ? &ext : nullptr;
+  Layout L = carve(o, pat, B, pb, ab, mode, external, static_cast<char*>(ws), &need, &q, use_stream, adaptive);
+  if (external && L.streaming && ws_bytes < need)  // room for the per-lane kernel only
+    L = carve(o, pat, B, pb, ab, mode, external, static_cast<char*>(ws), &need, &q, false, adaptive);
   if (ws == nullptr || ws_bytes < need)
     return fail(WMPC_ERR_WORKSPACE, "OSQP solve needs %zu workspace bytes, got %zu", need, ws_bytes);
   int rc;
@@ -1018,14 +1040,14 @@ int osqp_solve(const wmpc_osqp& q, const wmpc_osqp_options& opt, const wmpc_osqp
   }
   if (L.streaming && band_for(q, (B + 31) / 32)) {
     BandJobDesc job;
-    if ((rc = band_solve_begin(q, opt, d, L, &job, s))) return rc;
+    if ((rc = band_solve_begin(q, opt, d, L, &job, s, given))) return rc;
     if ((rc = band_run(&job, 1, L.error_word, q.num_sms, s))) return rc;
     return stream_solve_end(q, opt, d, L, nullptr, L.error_word, s);
   }
   if (L.streaming) {
     StreamJobDesc job;
     const bool frontier = frontier_for(q, opt.check_termination > 0, (B + 31) / 32);
-    if ((rc = stream_solve_begin(q, opt, d, L, frontier, &job, s))) return rc;
+    if ((rc = stream_solve_begin(q, opt, d, L, frontier, &job, s, given))) return rc;
     if ((rc = stream_run(&job, 1, L.error_word, q.num_sms, s))) return rc;
     return stream_solve_end(q, opt, d, L, &job, L.error_word, s);
   }
@@ -1061,7 +1083,6 @@ int osqp_solve(const wmpc_osqp& q, const wmpc_osqp_options& opt, const wmpc_osqp
     dinv = L.dinv;
     fb = kb;
   }
-  if (external && fb != 1 && fb != B) return fail(WMPC_ERR_INVALID_ARGUMENT, "factor_batch must be 1 or batch");
 
   if (mode == WMPC_OSQP_PLAIN) {
     const int fstride = fb > 1 ? 1 : 0;

@@ -51,6 +51,16 @@ struct Osqp {
 
 }  // namespace wmpc
 
+namespace wmpc {
+
+// a factorization given by the caller: lx [nnz_l, batch], dinv [n, batch]; batch 1: shared
+struct ExternalFactor {
+  const float *lx, *dinv;
+  int batch;
+};
+
+}  // namespace wmpc
+
 struct wmpc_osqp {
   int device = 0;
   int num_sms = 0;

@@ -1566,12 +1566,59 @@ int stream_factor(const Pattern& pat, const StreamPlan& sp, const Osqp& o, const
   return WMPC_OK;
 }
 
+// A given factorization (lx [nnz_l, fb], dinv [n, fb]; fb 1: shared by the
+// batch) into a schedule's streams: every entry where factor_stream_kernel would
+// have written it.  One block per tile, lane = instance; bound by the writes,
+// which are scattered 4-byte words of 16-byte units (L2 joins them).
+__global__ void __launch_bounds__(1024) factor_import_kernel(Pattern pat, StreamPlan sp, const float* __restrict__ lx,
+                                                             const float* __restrict__ dinv, int fb,
+                                                             float* __restrict__ bstream, float* __restrict__ fstream,
+                                                             int* __restrict__ status, int batch) {
+  __shared__ unsigned bad;  // lanes whose pivots are zero or not finite
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int b = blockIdx.x * 32 + lane;
+  const int fcol = fb > 1 ? (b < batch ? b : batch - 1) : 0;  // padding lanes copy the last instance
+  float* Lb = bstream + (size_t)blockIdx.x * sp.blen;
+  float* Lu = Lb + lane * 4;
+  float* F = fstream + (size_t)blockIdx.x * sp.flen + lane * 4;
+  if (threadIdx.x == 0) bad = 0;
+  __syncthreads();
+#pragma unroll 4
+  for (int e = warp; e < pat.nnz_l; e += warps) {
+    const float v = __ldg(lx + (size_t)__ldg(pat.proc_lidx + e) * fb + fcol);
+    Lu[__ldg(sp.proc_boff + e)] = v;
+    const int fo = __ldg(sp.proc_foff + e);
+    if (fo >= 0) F[fo] = v; else Lu[-1 - fo] = v;
+  }
+#pragma unroll 4
+  for (int k = warp; k < pat.n; k += warps) {
+    const float di = __ldg(dinv + (size_t)k * fb + fcol);
+    Lb[__ldg(&sp.row_info[2 * k + 1].z) + lane] = di;
+    const unsigned zero = __ballot_sync(kFullMask, di == 0.0f || !isfinite(di));
+    if (zero && lane == 0) atomicOr(&bad, zero);
+  }
+  for (int i = warp; i < sp.n_pad_b; i += warps) Lu[__ldg(sp.pad_boff + i)] = 0.0f;
+  for (int i = warp; i < sp.n_pad_f; i += warps) F[__ldg(sp.pad_foff + i)] = 0.0f;
+  __syncthreads();
+  if (warp == 0) status[b] = (bad >> lane & 1u) ? WMPC_STATUS_ZERO_PIVOT : 0;
+}
+
+int stream_import(const Pattern& pat, const StreamPlan& sp, const ExternalFactor& f, float* bstream, float* fstream,
+                  int* status, int batch, cudaStream_t s) {
+  profile_mark_begin(s, kProfileFactor);
+  factor_import_kernel<<<(batch + 31) / 32, 1024, 0, s>>>(pat, sp, f.lx, f.dinv, f.batch, bstream, fstream, status,
+                                                          batch);
+  profile_mark_end(s, kProfileFactor);
+  WMPC_LAUNCH_CHECK();
+  return WMPC_OK;
+}
+
 // Factorization into the streams and the state into its records (one class).
 int stream_begin(const Pattern& pat, const StreamPlan& sp, const Osqp& o, const float* pT, long long ldp, int sbp,
                  const float* aT, long long lda, int sba, const float* x, const float* z, const float* y,
                  const float* qs, const float* ls, const float* us, bool warm, bool track, float* work,
                  int* status, int batch, int num_sms, bool reuse_factor, StreamJobDesc* job, cudaStream_t s,
-                 const float* rinv_rows, const int* only) {
+                 const float* rinv_rows, const int* only, const ExternalFactor* given) {
   StreamLaunch cfg;
   if (!stream_launch_config(sp, &cfg)) return fail(WMPC_ERR_UNSUPPORTED, "pattern too large for the streaming kernel");
   const int n_tiles = (batch + 31) / 32;
@@ -1586,9 +1633,10 @@ int stream_begin(const Pattern& pat, const StreamPlan& sp, const Osqp& o, const 
   float* rhs = sp.frontier_slots > 0 ? pres + tl * sp.n : nullptr;
   float* fwd = sp.frontier_slots > 0 ? rhs + tl * sp.n : nullptr;
   OsqpInputs in{pT, ldp, sbp, aT, lda, sba, rinv_rows, rinv_rows ? (long long)batch : 0};
-  if (!reuse_factor) {
-    const int rc = stream_factor(pat, sp, o, pT, ldp, sbp, aT, lda, sba, bstream, fstream, status, batch, num_sms, s,
-                                 rinv_rows, only);
+  if (given || !reuse_factor) {
+    const int rc = given ? stream_import(pat, sp, *given, bstream, fstream, status, batch, s)
+                         : stream_factor(pat, sp, o, pT, ldp, sbp, aT, lda, sba, bstream, fstream, status, batch,
+                                         num_sms, s, rinv_rows, only);
     if (rc) return rc;
   }
   {
