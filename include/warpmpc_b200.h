@@ -361,6 +361,12 @@ int wmpc_stream_schedule_host(const wmpc_pattern_desc* desc, const float* rho, c
 int wmpc_band_tables_host(const wmpc_pattern_desc* desc, const float* rho, const float* rhoinv, int32_t n_primal,
                           int32_t* out, int64_t out_capacity, int64_t* out_words);
 
+/* The tile factorization's lists for a pattern whose inputs are the KKT values
+ * themselves and whose results go to L's entries in order and D^-1 by row
+ * (warpmpc_b200/csrc/tile_factor.cuh), built on the host: no device needed.
+ * out: [warps, delay, slots, ticks, words] warp_off[warps] prog[words]. */
+int wmpc_tile_factor_host(const wmpc_pattern_desc* desc, int32_t* out, int64_t out_capacity, int64_t* out_words);
+
 /* Profiling (no counterpart in the reference, which times with wall
  * clocks around jax.block_until_ready).  Between begin and end the library
  * records a CUDA event pair on the launching stream around every launch of

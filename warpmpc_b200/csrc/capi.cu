@@ -162,11 +162,26 @@ struct Packer {
 };
 
 
+// The factorization's lists (the plan's rho, per-instance rho; empty: not
+// available) placed for one stream layout and packed.
+void add_tile_factor(const int* boff, const int* foff, const int* doff, HostTileFactor* lists, TileFactor* out,
+                     Packer* pk) {
+  for (int i = 0; i < 2; ++i) {
+    out[i] = TileFactor{};
+    if (lists[i].prog.empty()) continue;
+    place_tile_factor(boff, foff, doff, &lists[i]);
+    pk->add(lists[i].prog.data(), lists[i].prog.size(), reinterpret_cast<const int**>(&out[i].prog));
+    pk->add(lists[i].warp_off.data(), lists[i].warp_off.size(), &out[i].warp_off);
+    out[i].slots = lists[i].slots;
+  }
+}
+
 // One streaming schedule of an OSQP problem: compact factor tables, chunk
 // schedule and launch check, uploaded in one block.  False (why set) when the
 // pattern cannot use the streaming kernel in this form.
 bool build_stream_plan(const HostPattern& hp, const StreamTargets& targets, const wmpc_osqp_desc* desc,
-                       const std::vector<float>& unscale, StreamPlan* out, void** block, std::string* why) {
+                       const std::vector<float>& unscale, StreamPlan* out, void** block, HostTileFactor* lists,
+                       TileFactor* tile_factor, std::string* why) {
   HostStream hs;
   std::vector<int> init_slot, upd_ptr;
   std::vector<unsigned short> upd_slot16;
@@ -262,6 +277,7 @@ bool build_stream_plan(const HostPattern& hp, const StreamTargets& targets, cons
   sk.add(hs.fmeta_off.data(), hs.fmeta_off.size(), &sp.fmeta_off);
   sk.add(hs.fmeta_words.data(), hs.fmeta_words.size(), &sp.fmeta_words);
   sk.add(hs.fmeta.data(), hs.fmeta.size(), &sp.fmeta);
+  add_tile_factor(hs.proc_boff.data(), hs.proc_foff.data(), hs.dinv_off.data(), lists, tile_factor, &sk);
   int* sblock = nullptr;
   if (sk.upload(&sblock) != WMPC_OK) {
     *why = g_last_error;
@@ -275,7 +291,8 @@ bool build_stream_plan(const HostPattern& hp, const StreamTargets& targets, cons
 // The band form of an OSQP problem: its tables, and the factorization tables
 // that write its stream.  False (why set) where the pattern has none.
 bool build_band_plan(const HostPattern& hp, const wmpc_osqp_desc* desc, const std::vector<float>& unscale,
-                     BandPlan* out, StreamPlan* factor, void** block, std::string* why) {
+                     BandPlan* out, StreamPlan* factor, void** block, HostTileFactor* lists, TileFactor* tile_factor,
+                     std::string* why) {
   HostBand hb;
   std::vector<int> init_slot, upd_ptr;
   std::vector<unsigned short> upd_slot16;
@@ -337,6 +354,7 @@ bool build_band_plan(const HostPattern& hp, const wmpc_osqp_desc* desc, const st
   sk.add(boff.data(), boff.size(), &sp.proc_boff);
   sk.add(foff.data(), foff.size(), &sp.proc_foff);
   sk.add(hb.pad.data(), hb.pad.size(), &sp.pad_boff);
+  add_tile_factor(boff.data(), foff.data(), hb.dpos.data(), lists, tile_factor, &sk);
   int* sblock = nullptr;
   if (sk.upload(&sblock) != WMPC_OK) {
     *why = g_last_error;
@@ -540,6 +558,54 @@ int wmpc_band_tables_host(const wmpc_pattern_desc* desc, const float* rho, const
   app(hb.item, hb.item.size()); app(hb.rec, hb.rec.size()); app(hb.rec_off, hb.rec_off.size());
   app(hb.iter_off, n); app(hb.param_off, n); app(hb.lpos, nnz_l); app(hb.lpos2, nnz_l); app(hb.dpos, n);
   app(hb.pad, hb.pad.size());
+  *out_words = static_cast<int64_t>(w.size());
+  if (!out) return WMPC_OK;
+  if (out_capacity < static_cast<int64_t>(w.size())) return fail(WMPC_ERR_INVALID_ARGUMENT, "output buffer too small");
+  std::memcpy(out, w.data(), w.size() * sizeof(int32_t));
+  return WMPC_OK;
+}
+
+int wmpc_tile_factor_host(const wmpc_pattern_desc* desc, int32_t* out, int64_t out_capacity, int64_t* out_words) {
+  if (!desc || !out_words) return fail(WMPC_ERR_INVALID_ARGUMENT, "null argument");
+  const int n = desc->n, nnz_l = desc->nnz_l;
+  if (n <= 0 || nnz_l < 0) return fail(WMPC_ERR_INVALID_ARGUMENT, "bad sizes");
+  HostPattern hp;
+  hp.n = n;
+  hp.nnz_a = desc->nnz_a;
+  hp.nnz_l = nnz_l;
+  const int n_init = desc->init_ptr[n], n_proc = desc->proc_ptr[n];
+  hp.init_ptr.assign(desc->init_ptr, desc->init_ptr + n + 1);
+  hp.init_rows.assign(desc->init_rows, desc->init_rows + n_init);
+  hp.proc_ptr.assign(desc->proc_ptr, desc->proc_ptr + n + 1);
+  hp.proc_cols.assign(desc->proc_cols, desc->proc_cols + n_proc);
+  hp.proc_offsets.assign(desc->proc_offsets, desc->proc_offsets + n_proc);
+  hp.proc_lidx.assign(desc->proc_lidx, desc->proc_lidx + n_proc);
+  hp.lp.assign(desc->lp, desc->lp + n + 1);
+  hp.li.assign(desc->li, desc->li + nnz_l);
+  hp.p.assign(desc->p, desc->p + n);
+  std::vector<int> init_slot, upd_ptr, boff(nnz_l), doff(n);
+  std::vector<unsigned short> upd_slot;
+  std::vector<int32_t> kin;
+  int max_row = 0;
+  const float one = 1.0f;
+  int32_t one_bits;
+  std::memcpy(&one_bits, &one, 4);
+  for (int k = 0; k < n; ++k) {  // the KKT values themselves
+    doff[k] = k;
+    kin.insert(kin.end(), {desc->perm_to_orig[desc->diag_pos[k]], 2, one_bits, 0});
+    for (int e = desc->init_ptr[k]; e < desc->init_ptr[k + 1]; ++e)
+      kin.insert(kin.end(), {desc->perm_to_orig[desc->init_pos[e]], 2, one_bits, 0});
+  }
+  for (int e = 0; e < nnz_l; ++e) boff[e] = hp.proc_lidx[e];
+  std::string why;
+  HostTileFactor t;
+  if (!build_factor_tables(hp, &init_slot, &upd_ptr, &upd_slot, &max_row, &why) ||
+      !build_tile_factor(hp, init_slot, kin.data(), desc->nnz_a, 0, &t, &why))
+    return fail(WMPC_ERR_UNSUPPORTED, "%s", why.c_str());
+  place_tile_factor(boff.data(), boff.data(), doff.data(), &t);
+  std::vector<int> w{kTfWarps, kTfDelay, t.slots, t.ticks, (int)t.prog.size()};
+  w.insert(w.end(), t.warp_off.begin(), t.warp_off.end());
+  w.insert(w.end(), t.prog.begin(), t.prog.end());
   *out_words = static_cast<int64_t>(w.size());
   if (!out) return WMPC_OK;
   if (out_capacity < static_cast<int64_t>(w.size())) return fail(WMPC_ERR_INVALID_ARGUMENT, "output buffer too small");
@@ -852,10 +918,11 @@ int wmpc_osqp_create(const wmpc_osqp_desc* desc, const wmpc_plan* kkt_plan, wmpc
   pk.add(p_up_rows.data(), np, &q->p_upper_rows);
   pk.add(p_up_cols.data(), np, &q->p_upper_cols);
   // the factorization rows' KKT inputs in row-program order, resolved
+  std::vector<int32_t> kin_base, kin_rho;
   {
     const wmpc_plan& kp = *kkt_plan;
     const int nkkt = n + m;
-    std::vector<int32_t> kin;
+    std::vector<int32_t>& kin = kin_base;
     kin.reserve(4 * ((size_t)nkkt + kp.h_init_pos.size()));
     auto put = [&](int slot) {
       const int idx = kp.h_perm_to_orig[slot];
@@ -903,7 +970,7 @@ int wmpc_osqp_create(const wmpc_osqp_desc* desc, const wmpc_plan* kkt_plan, wmpc
     // the factorization rows' inputs with every -1/rho slot read from the
     // instance's 1/rho row (constraint r: source nnz_p + nnz_a + r, kind 3)
     const wmpc_plan& kp = *kkt_plan;
-    std::vector<int32_t> kin;
+    std::vector<int32_t>& kin = kin_rho;
     kin.reserve(4 * ((size_t)(n + m) + kp.h_init_pos.size()));
     auto put = [&](int slot) {
       const int idx = kp.h_perm_to_orig[slot];
@@ -960,6 +1027,20 @@ int wmpc_osqp_create(const wmpc_osqp_desc* desc, const wmpc_plan* kkt_plan, wmpc
     hp.lp = kkt_plan->h_lp;
     hp.li = kkt_plan->h_li;
     hp.p = kkt_plan->h_p;
+    // the factorization's lists (WMPC_DISABLE_TILE_FACTOR: one warp per tile instead)
+    HostTileFactor lists[2];
+    if (!env_disabled("WMPC_DISABLE_TILE_FACTOR")) {
+      std::vector<int> init_slot, upd_ptr;
+      std::vector<unsigned short> upd_slot;
+      int max_row = 0;
+      std::string why;
+      if (build_factor_tables(hp, &init_slot, &upd_ptr, &upd_slot, &max_row, &why))
+        for (int i = 0; i < 2; ++i) {
+          const std::vector<int32_t>& kin = i ? kin_rho : kin_base;
+          if (!kin.empty() && !build_tile_factor(hp, init_slot, kin.data(), np, na, &lists[i], &why))
+            lists[i] = HostTileFactor{};
+        }
+    }
     StreamTargets targets;
     if (const char* v = getenv("WMPC_STREAM_UNITS")) targets.units = atoi(v);
     if (const char* v = getenv("WMPC_STREAM_COLS")) targets.cols = atoi(v);
@@ -981,10 +1062,11 @@ int wmpc_osqp_create(const wmpc_osqp_desc* desc, const wmpc_plan* kkt_plan, wmpc
     for (int j = 0; j < n; ++j) unscale[j] = desc->scaling_d[j];
     for (int r = 0; r < m; ++r) unscale[n + r] = std::max(desc->scaling_einv[r], desc->y_unscale[r]);
     q->has_stream = build_stream_plan(hp, frontier_mode == 1 ? ftargets : targets, desc, unscale, &q->sp,
-                                      &q->stream_block, &q->stream_why);
+                                      &q->stream_block, lists, q->tile_factor[0], &q->stream_why);
     if (q->has_stream && frontier_mode == 2) {
       std::string why;
-      q->has_frontier = build_stream_plan(hp, ftargets, desc, unscale, &q->spf, &q->stream_block_f, &why);
+      q->has_frontier = build_stream_plan(hp, ftargets, desc, unscale, &q->spf, &q->stream_block_f, lists,
+                                          q->tile_factor[1], &why);
       // worth it where it lets more CTAs share an SM than the plain form
       q->frontier_pays = q->has_frontier &&
                          stream_max_ctas(q->spf, kkt_plan->device, q->ctas_limit) >
@@ -992,7 +1074,8 @@ int wmpc_osqp_create(const wmpc_osqp_desc* desc, const wmpc_plan* kkt_plan, wmpc
     }
     std::string why;
     q->has_band = q->has_stream && band_wanted() &&
-                  build_band_plan(hp, desc, unscale, &q->bp, &q->band_factor, &q->band_block, &why);
+                  build_band_plan(hp, desc, unscale, &q->bp, &q->band_factor, &q->band_block, lists, q->tile_factor[2],
+                                  &why);
     if (q->has_band) q->band_tiles = band_tile_limit(q->bp, q->num_sms);
   }
   *out = q;

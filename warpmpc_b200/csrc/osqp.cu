@@ -719,12 +719,13 @@ int stream_begin(const Pattern& pat, const StreamPlan& sp, const Osqp& o, const 
                  const float* aT, long long lda, int sba, const float* x, const float* z, const float* y,
                  const float* qs, const float* ls, const float* us, bool warm, bool track, float* work,
                  int* status, int batch, int num_sms, bool reuse_factor, StreamJobDesc* job, cudaStream_t s,
-                 const float* rinv_rows = nullptr, const int* only = nullptr, const ExternalFactor* given = nullptr);
+                 const TileFactor* tf, const float* rinv_rows = nullptr, const int* only = nullptr, const ExternalFactor* given = nullptr);
 int stream_import(const Pattern& pat, const StreamPlan& sp, const ExternalFactor& f, float* bstream, float* fstream,
                   int* status, int batch, cudaStream_t s);
 int stream_factor(const Pattern& pat, const StreamPlan& sp, const Osqp& o, const float* pT, long long ldp, int sbp,
                   const float* aT, long long lda, int sba, float* bstream, float* fstream, int* status, int batch,
-                  int num_sms, cudaStream_t s, const float* rinv_rows = nullptr, const int* only = nullptr);
+                  int num_sms, cudaStream_t s, const TileFactor* tf, const float* rinv_rows = nullptr,
+                  const int* only = nullptr);
 int stream_run(const StreamJobDesc* jobs, int n_jobs, int* error, int num_sms, cudaStream_t s);
 int stream_end(const StreamPlan& sp, const Osqp& o, const StreamJobDesc& job, float* x, float* z, float* y,
                cudaStream_t s);
@@ -833,7 +834,8 @@ int stream_solve_begin(const wmpc_osqp& q, const wmpc_osqp_options& opt, const w
   if ((rc = stream_begin(q.kkt_plan->pat, frontier ? q.spf : q.sp, o, L.pT, pb, pb > 1 ? 1 : 0, L.aT, ab, ab > 1 ? 1 : 0,
                          L.x, L.z, L.y,
                          L.qs, L.ls, L.us, opt.warm_start != 0, check > 0, L.stream_ws, L.stream_status, B,
-                         q.num_sms, opt.reuse_factor != 0, job, s, nullptr, nullptr, given)))
+                         q.num_sms, opt.reuse_factor != 0, job, s, q.tile_factor[frontier ? 1 : 0], nullptr, nullptr,
+                         given)))
     return rc;
   // termination: an instance stops (freezes) once both its primal residual
   // (A x - z, carried exactly through the iterations) and its largest iterate
@@ -865,7 +867,7 @@ int band_prepare(const wmpc_osqp& q, const wmpc_osqp_options& opt, const wmpc_os
       return rc;
   } else if (!reuse_factor &&
       (rc = stream_factor(q.kkt_plan->pat, q.band_factor, o, L.pT, pb, pb > 1 ? 1 : 0, L.aT, ab, ab > 1 ? 1 : 0,
-                          w.stream, w.stream, L.stream_status, B, q.num_sms, s, rinv_rows, only)))
+                          w.stream, w.stream, L.stream_status, B, q.num_sms, s, q.tile_factor[2], rinv_rows, only)))
     return rc;
   if ((rc = band_state_in(q.bp, o, L.aT, ab, ab > 1 ? 1 : 0, check > 0, warm, L.x, L.z, L.y, L.qs, L.ls, L.us, w, B,
                           s)))
@@ -929,7 +931,8 @@ int stream_solve_adaptive(const wmpc_osqp& q, const wmpc_osqp_options& opt, cons
       return r;
     }
     int r = stream_begin(q.kkt_plan->pat, sp, o, L.pT, pb, sbp, L.aT, ab, sba, L.x, L.z, L.y, L.qs, L.ls, L.us, warm,
-                         false, L.stream_ws, L.stream_status, B, q.num_sms, false, job, s, L.rinv_row, only);
+                         false, L.stream_ws, L.stream_status, B, q.num_sms, false, job, s, q.tile_factor[frontier ? 1 : 0],
+                         L.rinv_row, only);
     job->check_every = 0;
     job->ctas_limit = q.ctas_limit;
     job->chg_eps = opt.eps_abs;

@@ -4,6 +4,7 @@
 #include "band.cuh"
 #include "common.cuh"
 #include "stream.cuh"
+#include "tile_factor.cuh"
 
 namespace wmpc {
 
@@ -84,5 +85,8 @@ struct wmpc_osqp {
   wmpc::BandPlan bp{};
   wmpc::StreamPlan band_factor{};  // the factorization's tables, writing the band form's stream
   void* band_block = nullptr;
+  // the factorization's lists for the plain, frontier and band streams, with the
+  // plan's and with per-instance rho
+  wmpc::TileFactor tile_factor[3][2];
   std::string stream_why;  // why the streaming path is unavailable (diagnostics)
 };

@@ -1537,10 +1537,17 @@ size_t stream_workspace_floats(const StreamPlan& sp, int batch) {
 // 1/rho inputs; only: just the tiles holding a marked instance).
 int stream_factor(const Pattern& pat, const StreamPlan& sp, const Osqp& o, const float* pT, long long ldp, int sbp,
                   const float* aT, long long lda, int sba, float* bstream, float* fstream, int* status, int batch,
-                  int num_sms, cudaStream_t s, const float* rinv_rows, const int* only) {
+                  int num_sms, cudaStream_t s, const TileFactor* tf, const float* rinv_rows, const int* only) {
   const int n_tiles = (batch + 31) / 32;
   OsqpInputs in{pT, ldp, sbp, aT, lda, sba, rinv_rows, rinv_rows ? (long long)batch : 0};
   if (rinv_rows && !o.kin_desc_rho) return fail(WMPC_ERR_UNSUPPORTED, "the problem has no per-instance rho inputs");
+  // the tile kernel wherever its lists could be built (faster from one tile to
+  // thousands; figures there): else, for columns or values in flight past its
+  // bounds, one warp per tile
+  const TileFactor& lists = tf[rinv_rows ? 1 : 0];
+  if (lists.prog)
+    return tile_factor_stream(lists, sp, TileFactorInputs{pT, aT, rinv_rows, ldp, lda, in.ldr, sbp, sba, o.nnz_p, o.nnz_a},
+                              bstream, fstream, status, batch, num_sms, only, s);
   // L-batch sized so that every tile's warp is resident at once (all of a
   // launch's rows then wait out their round trips together)
   const int warps = 2;
@@ -1618,7 +1625,7 @@ int stream_begin(const Pattern& pat, const StreamPlan& sp, const Osqp& o, const 
                  const float* aT, long long lda, int sba, const float* x, const float* z, const float* y,
                  const float* qs, const float* ls, const float* us, bool warm, bool track, float* work,
                  int* status, int batch, int num_sms, bool reuse_factor, StreamJobDesc* job, cudaStream_t s,
-                 const float* rinv_rows, const int* only, const ExternalFactor* given) {
+                 const TileFactor* tf, const float* rinv_rows, const int* only, const ExternalFactor* given) {
   StreamLaunch cfg;
   if (!stream_launch_config(sp, &cfg)) return fail(WMPC_ERR_UNSUPPORTED, "pattern too large for the streaming kernel");
   const int n_tiles = (batch + 31) / 32;
@@ -1636,7 +1643,7 @@ int stream_begin(const Pattern& pat, const StreamPlan& sp, const Osqp& o, const 
   if (given || !reuse_factor) {
     const int rc = given ? stream_import(pat, sp, *given, bstream, fstream, status, batch, s)
                          : stream_factor(pat, sp, o, pT, ldp, sbp, aT, lda, sba, bstream, fstream, status, batch,
-                                         num_sms, s, rinv_rows, only);
+                                         num_sms, s, tf, rinv_rows, only);
     if (rc) return rc;
   }
   {

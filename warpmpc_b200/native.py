@@ -266,6 +266,8 @@ SIGNATURES = {
     "wmpc_quadrotor_jac_pattern": (ctypes.c_int, [_i32p, _i32p]),
     "wmpc_solve_tables_host": (ctypes.c_int, [ctypes.POINTER(PatternDesc), _i32p, ctypes.c_int64,
                                               ctypes.POINTER(ctypes.c_int64)]),
+    "wmpc_tile_factor_host": (ctypes.c_int, [ctypes.POINTER(PatternDesc), _i32p, ctypes.c_int64,
+                                             ctypes.POINTER(ctypes.c_int64)]),
     "wmpc_band_tables_host": (
         ctypes.c_int,
         [ctypes.POINTER(PatternDesc), _f32p, _f32p, ctypes.c_int32, _i32p, ctypes.c_int64,

@@ -84,6 +84,23 @@ def band_tables(plan) -> dict | None:
     return out
 
 
+def tile_factor_lists(qp) -> dict | None:
+    """The tile factorization's lists of a QDLDL plan
+    (``wmpc_tile_factor_host``), or None where the pattern has none."""
+    desc, keep, _ = _pattern_desc(qp)
+    lib = native.lib()
+    words = ctypes.c_int64()
+    rc = lib.wmpc_tile_factor_host(ctypes.byref(desc), None, 0, ctypes.byref(words))
+    if rc == native.WMPC_ERR_UNSUPPORTED:
+        return None
+    native.check(rc)
+    buf = np.empty(words.value, dtype=np.int32)
+    native.check(lib.wmpc_tile_factor_host(ctypes.byref(desc), native.ptr_i32(buf), buf.size, ctypes.byref(words)))
+    out = {k: int(v) for k, v in zip(("warps", "delay", "slots", "ticks", "words"), buf)}
+    out["warp_off"], out["prog"] = buf[5 : 5 + out["warps"]].copy(), buf[5 + out["warps"] :].reshape(-1, 4).copy()
+    return out
+
+
 def stream_schedule(plan, targets=DEFAULT_TARGETS) -> dict:
     """Schedule of an OSQP plan (rho per constraint) as NumPy arrays.
 
