@@ -421,19 +421,27 @@ __device__ __forceinline__ bool finite_res(const Residuals& r) {
 // order, so prim, dual and the norms (maxima) equal residuals()' exactly; the
 // objective's two sums are added part by part.  Eight times the warps in
 // flight for a latency-bound loop of dependent index and value loads.
-__global__ void __launch_bounds__(32 * kResParts) residual_kernel(
+// kSplit > 1: each part's rows and columns are dealt to kSplit threads, and the
+// first of them adds the objective's terms in the part's order (a round of
+// kResParts * kSplit columns at a time): the same bits.
+template <int kSplit>
+__global__ void __launch_bounds__(32 * kResParts * kSplit) residual_kernel(
     Osqp o, const float* __restrict__ pT, long long ldp, int sbp, const float* __restrict__ aT, long long lda,
     int sba, State st, const float* __restrict__ qT, float* prim, float* dual, float* obj, int* status, int batch,
     const int* status_in, const int* abort_word, float eps_abs, float eps_rel) {
-  __shared__ float part_val[kResParts][9][32];
+  constexpr int kAll = kResParts * kSplit;
+  __shared__ float part_val[kAll][9][32];
+  // two rounds' objective terms, in the same memory
+  auto terms = reinterpret_cast<float (*)[kAll][2][32]>(&part_val[0][0][0]);
   const int lane = threadIdx.x, part = threadIdx.y;
   const int b = blockIdx.x * 32 + lane;
   const bool active = b < batch;
-  if (active) {
+  {
+    const int b = active ? blockIdx.x * 32 + lane : batch - 1;  // (idle lanes keep the rounds' barriers)
     InstanceData in{pT + (long long)b * sbp, ldp, aT + (long long)b * sba, lda};
     auto xu = [&](int j) { return st.x[(long long)j * st.ld + b] * __ldg(o.scaling_d + j); };
     float rp = 0.f, axn = 0.f, zn = 0.f;
-    for (int row = part; row < o.m; row += kResParts) {
+    for (int row = part; row < o.m; row += kAll) {
       float ax = 0.0f;
       const int e0 = __ldg(o.a_row_ptr + row), e1 = __ldg(o.a_row_ptr + row + 1);
 #pragma unroll 4
@@ -447,28 +455,46 @@ __global__ void __launch_bounds__(32 * kResParts) residual_kernel(
       zn = fmaxf(zn, fabsf(zu));
     }
     float rd = 0.f, pxn = 0.f, atyn = 0.f, qn = 0.f, quad = 0.f, lin = 0.f;
-    for (int j = part; j < o.n; j += kResParts) {
-      float px = 0.0f;
-      const int f0 = __ldg(o.pf_row_ptr + j), f1 = __ldg(o.pf_row_ptr + j + 1);
+    for (int j0 = 0; j0 < o.n; j0 += kAll) {
+      const int j = j0 + part;
+      float px = 0.0f, qj = 0.0f, xj = 0.0f;
+      if (j < o.n) {
+        const int f0 = __ldg(o.pf_row_ptr + j), f1 = __ldg(o.pf_row_ptr + j + 1);
 #pragma unroll 4
-      for (int t = f0; t < f1; ++t) px = px + in.p(__ldg(o.pf_val + t)) * xu(__ldg(o.pf_col + t));
-      float aty = 0.0f;
-      const int c0 = __ldg(o.a_col_ptr + j), c1 = __ldg(o.a_col_ptr + j + 1);
+        for (int t = f0; t < f1; ++t) px = px + in.p(__ldg(o.pf_val + t)) * xu(__ldg(o.pf_col + t));
+        float aty = 0.0f;
+        const int c0 = __ldg(o.a_col_ptr + j), c1 = __ldg(o.a_col_ptr + j + 1);
 #pragma unroll 4
-      for (int e = c0; e < c1; ++e) {
-        const int row = __ldg(o.a_rows + e);
-        aty = aty + in.a(e) * (st.y[(long long)row * st.ld + b] * __ldg(o.y_unscale + row));
+        for (int e = c0; e < c1; ++e) {
+          const int row = __ldg(o.a_rows + e);
+          aty = aty + in.a(e) * (st.y[(long long)row * st.ld + b] * __ldg(o.y_unscale + row));
+        }
+        qj = qT[(long long)j * batch + b];
+        xj = xu(j);
+        rd = fmaxf(rd, fabsf(px + qj + aty));
+        pxn = fmaxf(pxn, fabsf(px));
+        atyn = fmaxf(atyn, fabsf(aty));
+        qn = fmaxf(qn, fabsf(qj));
       }
-      const float qj = qT[(long long)j * batch + b];
-      const float xj = xu(j);
-      rd = fmaxf(rd, fabsf(px + qj + aty));
-      pxn = fmaxf(pxn, fabsf(px));
-      atyn = fmaxf(atyn, fabsf(aty));
-      qn = fmaxf(qn, fabsf(qj));
-      quad = quad + xj * px;
-      lin = lin + qj * xj;
+      if constexpr (kSplit == 1) {
+        if (j < o.n) {
+          quad = quad + xj * px;
+          lin = lin + qj * xj;
+        }
+      } else {
+        const int round = (j0 / kAll) & 1;
+        terms[round][part][0][lane] = xj * px;
+        terms[round][part][1][lane] = qj * xj;
+        __syncthreads();
+        if (part < kResParts)
+          for (int i = part; i < kAll && j0 + i < o.n; i += kResParts) {
+            quad = quad + terms[round][i][0][lane];
+            lin = lin + terms[round][i][1][lane];
+          }
+      }
     }
     const float v[9] = {rp, axn, zn, rd, pxn, atyn, qn, quad, lin};
+    if constexpr (kSplit > 1) __syncthreads();
 #pragma unroll
     for (int k = 0; k < 9; ++k) part_val[part][k][lane] = v[k];
   }
@@ -476,7 +502,7 @@ __global__ void __launch_bounds__(32 * kResParts) residual_kernel(
   if (active && part == 0) {
     Residuals r{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     float quad = 0.f, lin = 0.f;
-    for (int q = 0; q < kResParts; ++q) {
+    for (int q = 0; q < kAll; ++q) {
       r.prim = fmaxf(r.prim, part_val[q][0][lane]);
       r.ax_norm = fmaxf(r.ax_norm, part_val[q][1][lane]);
       r.z_norm = fmaxf(r.z_norm, part_val[q][2][lane]);
@@ -484,6 +510,7 @@ __global__ void __launch_bounds__(32 * kResParts) residual_kernel(
       r.px_norm = fmaxf(r.px_norm, part_val[q][4][lane]);
       r.aty_norm = fmaxf(r.aty_norm, part_val[q][5][lane]);
       r.q_norm = fmaxf(r.q_norm, part_val[q][6][lane]);
+      if (q >= kResParts) continue;
       quad = quad + part_val[q][7][lane];
       lin = lin + part_val[q][8][lane];
     }
@@ -504,15 +531,32 @@ __global__ void __launch_bounds__(32 * kResParts) residual_kernel(
     }
   }
   if (!active) return;
-  for (int j = part; j < o.n; j += kResParts) {
+  for (int j = part; j < o.n; j += kAll) {
     const long long k = (long long)j * st.ld + b;
     st.x[k] = st.x[k] * __ldg(o.scaling_d + j);
   }
-  for (int r = part; r < o.m; r += kResParts) {
+  for (int r = part; r < o.m; r += kAll) {
     const long long k = (long long)r * st.ld + b;
     st.z[k] = st.z[k] * __ldg(o.scaling_einv + r);
     st.y[k] = st.y[k] * __ldg(o.y_unscale + r);
   }
+}
+
+// Four threads per part up to two tiles per SM, where the loop's latency is what
+// the kernel takes (us: one 30-step quadrotor instance 173 to 79, 1000 of them 396
+// to 135); with more tiles one thread per part fills the SMs (65,536 instances of
+// the 10-step 6-state class 165, split 231).
+void launch_residual(const Osqp& o, const float* pT, long long ldp, int sbp, const float* aT, long long lda, int sba,
+                     const State& st, const float* qT, float* prim, float* dual, float* obj, int* status, int batch,
+                     const int* status_in, const int* abort_word, float eps_abs, float eps_rel, int num_sms,
+                     cudaStream_t s) {
+  const int tiles = ceil_div(batch, 32);
+  if (tiles <= 2 * num_sms)
+    residual_kernel<4><<<tiles, dim3(32, 4 * kResParts), 0, s>>>(o, pT, ldp, sbp, aT, lda, sba, st, qT, prim, dual, obj,
+                                                                 status, batch, status_in, abort_word, eps_abs, eps_rel);
+  else
+    residual_kernel<1><<<tiles, dim3(32, kResParts), 0, s>>>(o, pT, ldp, sbp, aT, lda, sba, st, qT, prim, dual, obj,
+                                                             status, batch, status_in, abort_word, eps_abs, eps_rel);
 }
 
 // The final iterate's unscaling alone (no residual outputs requested): x,
@@ -1008,9 +1052,8 @@ int stream_solve_end(const wmpc_osqp& q, const wmpc_osqp_options& opt, const wmp
     return rc;
   State st{L.x, L.z, L.y, L.qs, L.ls, L.us, B};
   if (residuals_wanted(opt, d)) {
-    residual_kernel<<<ceil_div(B, 32), dim3(32, kResParts), 0, s>>>(
-        o, L.pT, pb, pb > 1 ? 1 : 0, L.aT, ab, ab > 1 ? 1 : 0, st, L.qT, d.prim_res, d.dual_res, d.obj, d.status, B,
-        L.stream_status, error_word, check ? opt.eps_abs : -1.0f, opt.eps_rel);
+    launch_residual(o, L.pT, pb, pb > 1 ? 1 : 0, L.aT, ab, ab > 1 ? 1 : 0, st, L.qT, d.prim_res, d.dual_res, d.obj,
+                    d.status, B, L.stream_status, error_word, check ? opt.eps_abs : -1.0f, opt.eps_rel, q.num_sms, s);
   } else {
     unscale_state_kernel<<<ceil_div(B, 32), dim3(32, kResParts), 0, s>>>(o, st, d.status, L.stream_status, error_word, B);
   }
@@ -1151,9 +1194,8 @@ int osqp_solve(const wmpc_osqp& q, const wmpc_osqp_options& opt, const wmpc_osqp
       WMPC_LAUNCH_CHECK();
     }
     if (residuals_wanted(opt, d)) {
-      residual_kernel<<<ceil_div(B, 32), dim3(32, kResParts), 0, s>>>(
-          o, L.pT, ldp, sbp, L.aT, lda, sba, st, L.qT, d.prim_res, d.dual_res, d.obj, d.status, B, nullptr, nullptr,
-          -1.0f, 0.0f);
+      launch_residual(o, L.pT, ldp, sbp, L.aT, lda, sba, st, L.qT, d.prim_res, d.dual_res, d.obj, d.status, B, nullptr,
+                      nullptr, -1.0f, 0.0f, q.num_sms, s);
     } else {
       unscale_state_kernel<<<ceil_div(B, 32), dim3(32, kResParts), 0, s>>>(o, st, d.status, nullptr, nullptr, B);
     }
