@@ -599,8 +599,10 @@ int wmpc_tile_factor_host(const wmpc_pattern_desc* desc, int32_t* out, int64_t o
   for (int e = 0; e < nnz_l; ++e) boff[e] = hp.proc_lidx[e];
   std::string why;
   HostTileFactor t;
+  HostTileSchedule sched;
   if (!build_factor_tables(hp, &init_slot, &upd_ptr, &upd_slot, &max_row, &why) ||
-      !build_tile_factor(hp, init_slot, kin.data(), desc->nnz_a, 0, &t, &why))
+      !schedule_tile_factor(hp, init_slot, &sched, &why) ||
+      !emit_tile_factor(sched, hp, init_slot, kin.data(), desc->nnz_a, 0, &t, &why))
     return fail(WMPC_ERR_UNSUPPORTED, "%s", why.c_str());
   place_tile_factor(boff.data(), boff.data(), doff.data(), &t);
   std::vector<int> w{kTfWarps, kTfDelay, t.slots, t.ticks, (int)t.prog.size()};
@@ -676,6 +678,7 @@ int wmpc_plan_create(const wmpc_pattern_desc* desc, int device, wmpc_plan** out)
   pk.add(desc->pinv, n, &pat.pinv);
   // compact-accumulator tables of the staged per-call factorization
   std::vector<int> fac_init_slot, fac_upd_ptr, fac_upd_slot, fac_upd_lidx;
+  HostTileFactor tile;
   {
     HostPattern hp;
     hp.n = n;
@@ -717,6 +720,25 @@ int wmpc_plan_create(const wmpc_pattern_desc* desc, int device, wmpc_plan** out)
       pk.add(kin_slot.data(), kin_slot.size(), &plan->fac_kin_slot);
       plan->fac_max_row = std::max(max_row, 1);
       plan->fac_max_kv = max_kv;
+      // the tile factorization (WMPC_DISABLE_TILE_FACTOR: one warp per tile instead)
+      auto sched = std::make_shared<HostTileSchedule>();
+      if (!env_disabled("WMPC_DISABLE_TILE_FACTOR") && schedule_tile_factor(hp, fac_init_slot, sched.get(), &why)) {
+        const float one = 1.0f;
+        int32_t one_bits;
+        std::memcpy(&one_bits, &one, 4);
+        std::vector<int32_t> kin;  // the KKT values themselves
+        for (int slot : kin_slot) kin.insert(kin.end(), {slot, 2, one_bits, 0});
+        std::vector<int> doff(n);
+        for (int k = 0; k < n; ++k) doff[k] = k;
+        if (emit_tile_factor(*sched, hp, fac_init_slot, kin.data(), nnz_a, 0, &tile, &why)) {
+          place_tile_factor(hp.proc_lidx.data(), hp.proc_lidx.data(), doff.data(), &tile);
+          pk.add(tile.prog.data(), tile.prog.size(), reinterpret_cast<const int**>(&plan->tile_prog));
+          pk.add(tile.warp_off.data(), tile.warp_off.size(), &plan->tile_off);
+          plan->tile_slots = tile.slots;
+          plan->h_tile = sched;
+          plan->h_init_slot = fac_init_slot;
+        }
+      }
     }
   }
   // chunk tables of the TMA-fed per-call solve (when every column fits a chunk)
@@ -1027,19 +1049,16 @@ int wmpc_osqp_create(const wmpc_osqp_desc* desc, const wmpc_plan* kkt_plan, wmpc
     hp.lp = kkt_plan->h_lp;
     hp.li = kkt_plan->h_li;
     hp.p = kkt_plan->h_p;
-    // the factorization's lists (WMPC_DISABLE_TILE_FACTOR: one warp per tile instead)
+    // the factorization's lists
     HostTileFactor lists[2];
-    if (!env_disabled("WMPC_DISABLE_TILE_FACTOR")) {
-      std::vector<int> init_slot, upd_ptr;
-      std::vector<unsigned short> upd_slot;
-      int max_row = 0;
+    if (kkt_plan->h_tile) {
       std::string why;
-      if (build_factor_tables(hp, &init_slot, &upd_ptr, &upd_slot, &max_row, &why))
-        for (int i = 0; i < 2; ++i) {
-          const std::vector<int32_t>& kin = i ? kin_rho : kin_base;
-          if (!kin.empty() && !build_tile_factor(hp, init_slot, kin.data(), np, na, &lists[i], &why))
-            lists[i] = HostTileFactor{};
-        }
+      for (int i = 0; i < 2; ++i) {
+        const std::vector<int32_t>& kin = i ? kin_rho : kin_base;
+        if (!kin.empty() && !emit_tile_factor(*kkt_plan->h_tile, hp, kkt_plan->h_init_slot, kin.data(), np, na,
+                                              &lists[i], &why))
+          lists[i] = HostTileFactor{};
+      }
     }
     StreamTargets targets;
     if (const char* v = getenv("WMPC_STREAM_UNITS")) targets.units = atoi(v);

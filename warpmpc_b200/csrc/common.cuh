@@ -103,7 +103,12 @@ inline bool env_disabled(const char* name) {
 
 }  // namespace wmpc
 
+#include <memory>
 #include <vector>
+
+namespace wmpc {
+struct HostTileSchedule;
+}
 
 struct wmpc_plan {
   int device = 0;
@@ -118,6 +123,12 @@ struct wmpc_plan {
   // the one-lane kernel factors): slot of each initial entry in its row's
   // reach, per program entry its range of updates, per update its target
   // slot and the L entry it re-reads
+  // the tile factorization (tile_factor.cuh): its lists for the per-call factor, its schedule
+  const int4* tile_prog = nullptr;
+  const int* tile_off = nullptr;
+  int tile_slots = 0;
+  std::shared_ptr<wmpc::HostTileSchedule> h_tile;
+  std::vector<int> h_init_slot;
   const int* fac_init_slot = nullptr;
   const int* fac_upd_ptr = nullptr;
   const int* fac_upd_slot = nullptr;

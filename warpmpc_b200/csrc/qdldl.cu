@@ -15,6 +15,7 @@
 #include "common.cuh"
 #include "qdldl.cuh"
 #include "stream.cuh"
+#include "tile_factor.cuh"
 
 namespace wmpc {
 
@@ -298,6 +299,9 @@ int launch_factor_plan(const wmpc_plan& plan, const float* values, long long ldv
       (void)cudaGetLastError();
       num_sms = 148;
     }
+    if (plan.tile_prog)
+      return tile_factor_planes(TileFactor{plan.tile_prog, plan.tile_off, plan.tile_slots}, values, ldv, bstride, lx, d,
+                                dinv, batch, num_sms, only, stream);
     const int warps = 2;
     const int n_tiles = (batch + 31) / 32;
     // L-batch sized so that every tile's warp can be resident at once

@@ -1,5 +1,7 @@
 // Factorization of 32-instance tiles, one CTA per tile (sm_100a); the program it
 // runs is described in tile_factor.cuh.
+#include <climits>
+
 #include "osqp.cuh"
 #include "tile_factor.cuh"
 
@@ -68,7 +70,7 @@ tile_factor_kernel(TileFactor tf, TileFactorOut out, const float* __restrict__ s
     const float* pin = src_p + (long long)bb * sbp;
     const float* ain = src_a + (long long)bb * sba;
     const float* rin = src_r + (src_r ? bb : 0);
-    const bool write = !kPlanes || b < batch;
+    const bool write = !kPlanes || (b < batch && (only == nullptr || only[b] != 0));
     float* Lu = kPlanes ? out.b + b : out.b + (size_t)tile * out.tile_b + lane * 4;
     float* F = kPlanes ? nullptr : out.f + (size_t)tile * out.tile_f + lane * 4;
     float* Ld = kPlanes ? out.d + b : out.d + (size_t)tile * out.tile_d + lane;
@@ -203,23 +205,47 @@ tile_factor_kernel(TileFactor tf, TileFactorOut out, const float* __restrict__ s
   }
 }
 
-int tile_factor_stream(const TileFactor& tf, const StreamPlan& sp, const TileFactorInputs& in, float* bstream,
-                       float* fstream, int* status, int batch, int num_sms, const int* only, cudaStream_t s) {
-  const int n_tiles = (batch + 31) / 32;
-  const size_t smem = tile_factor_smem(tf.slots);
+static int tile_factor_launch(int slots, int n_tiles, int num_sms, int* grid, size_t* smem) {
+  *smem = tile_factor_smem(slots);
   int dev = 0, sm_bytes = 0, reserved = 0;
   WMPC_CUDA_TRY(cudaGetDevice(&dev));
   WMPC_CUDA_TRY(cudaDeviceGetAttribute(&sm_bytes, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
   WMPC_CUDA_TRY(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev));
-  const int per_sm = 2 * (smem + reserved + 1024) <= (size_t)sm_bytes ? 2 : 1;
+  const int most = num_sms * (2 * (*smem + reserved + 1024) <= (size_t)sm_bytes ? 2 : 1);
+  *grid = n_tiles < most ? n_tiles : most;
+  return WMPC_OK;
+}
+
+int tile_factor_stream(const TileFactor& tf, const StreamPlan& sp, const TileFactorInputs& in, float* bstream,
+                       float* fstream, int* status, int batch, int num_sms, const int* only, cudaStream_t s) {
+  const int n_tiles = (batch + 31) / 32;
+  int grid = 0;
+  size_t smem = 0;
+  if (int rc = tile_factor_launch(tf.slots, n_tiles, num_sms, &grid, &smem)) return rc;
   auto kernel = tile_factor_kernel<false>;
   WMPC_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const TileFactorOut out{bstream, fstream, bstream, sp.blen, sp.flen, sp.blen, nullptr, 0};
-  const int grid = n_tiles < per_sm * num_sms ? n_tiles : per_sm * num_sms;
   profile_mark_begin(s, kProfileFactor);
   kernel<<<grid, 32 * kTfWarps, smem, s>>>(tf, out, in.p, in.ldp, in.sbp, in.np, in.a, in.lda, in.sba, in.na, in.r,
                                            in.ldr, sp.pad_boff, sp.n_pad_b, sp.pad_foff, sp.n_pad_f, status, n_tiles,
                                            batch, only);
+  profile_mark_end(s, kProfileFactor);
+  WMPC_LAUNCH_CHECK();
+  return WMPC_OK;
+}
+
+int tile_factor_planes(const TileFactor& tf, const float* values, long long ld, int sb, float* lx, float* d,
+                       float* dinv, int batch, int num_sms, const int* only, cudaStream_t s) {
+  const int n_tiles = (batch + 31) / 32;
+  const TileFactorOut out{lx, nullptr, dinv, 0, 0, 0, d, batch};
+  int grid = 0;
+  size_t smem = 0;
+  auto kernel = tile_factor_kernel<true>;
+  if (int rc = tile_factor_launch(tf.slots, n_tiles, num_sms, &grid, &smem)) return rc;
+  WMPC_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  profile_mark_begin(s, kProfileFactor);
+  kernel<<<grid, 32 * kTfWarps, smem, s>>>(tf, out, values, ld, sb, INT_MAX, values, 0, 0, 0, nullptr, 0, nullptr, 0,
+                                           nullptr, 0, nullptr, n_tiles, batch, only);
   profile_mark_end(s, kProfileFactor);
   WMPC_LAUNCH_CHECK();
   return WMPC_OK;

@@ -56,6 +56,20 @@ struct TileFactor {
   int slots = 0;
 };
 
+// The schedule of a pattern: which warp does what in which tick, and the slots.
+struct HostTileSchedule {
+  struct Op {
+    int tick, task;  // task: step, nnz_l + row: init, nnz_l + n + row: load
+  };
+  std::vector<std::vector<Op>> ops;  // by warp
+  std::vector<int> slot;             // by step (its row's entry), then by row (d, then D^-1)
+  std::vector<std::vector<std::pair<int, int>>> upd;  // by step: {slot index in the row, the earlier row's step}
+  int slots = 0, ticks = 0;
+};
+
+bool schedule_tile_factor(const HostPattern& hp, const std::vector<int>& init_slot, HostTileSchedule* out,
+                          std::string* why);
+
 struct HostTileFactor {
   std::vector<int> prog, warp_off;
   std::vector<int> step_at, row_at;  // words of prog that hold a step's L offsets (two), a row's D^-1 offset
@@ -65,8 +79,8 @@ struct HostTileFactor {
 // The lists, without the places of the results.  kin: [n + inputs] {source or -1,
 // kind, scale, add} in row-program order, sources: np P values, na A values, then
 // 1/rho rows.
-bool build_tile_factor(const HostPattern& hp, const std::vector<int>& init_slot, const int* kin, int np, int na,
-                       HostTileFactor* out, std::string* why);
+bool emit_tile_factor(const HostTileSchedule& sched, const HostPattern& hp, const std::vector<int>& init_slot,
+                      const int* kin, int np, int na, HostTileFactor* out, std::string* why);
 
 // The places: boff, foff [nnz_l] by program step, doff [n].
 void place_tile_factor(const int* boff, const int* foff, const int* doff, HostTileFactor* t);
@@ -79,6 +93,11 @@ struct TileFactorInputs {
 };
 int tile_factor_stream(const TileFactor& tf, const StreamPlan& sp, const TileFactorInputs& in, float* bstream,
                        float* fstream, int* status, int batch, int num_sms, const int* only, cudaStream_t s);
+
+// Runs it over a batch of KKT values ([nnz][ld], batch stride sb), into lx [nnz_l][batch],
+// d and dinv [n][batch] (only: just the instances marked in it).
+int tile_factor_planes(const TileFactor& tf, const float* values, long long ld, int sb, float* lx, float* d,
+                       float* dinv, int batch, int num_sms, const int* only, cudaStream_t s);
 
 size_t tile_factor_smem(int slots);
 

@@ -35,16 +35,12 @@ void place_tile_factor(const int* boff, const int* foff, const int* doff, HostTi
   for (size_t k = 0; k < t->row_at.size(); ++k) t->prog[t->row_at[k]] = doff[k];
 }
 
-// look: rows start this far (in estimated cycles) ahead of the schedule
-static bool schedule_tile_factor(const HostPattern& hp, const std::vector<int>& init_slot, const int* kin, int np,
-                                 int na, int look, int max_slots, HostTileFactor* out, std::string* why) {
-  HostTileFactor& H = *out;
-  H = HostTileFactor{};
+bool schedule_tile_factor(const HostPattern& hp, const std::vector<int>& init_slot, HostTileSchedule* out,
+                          std::string* why) {
   const int n = hp.n, S = hp.nnz_l, N = S + n;  // tasks: steps, then the rows' inits
-  std::vector<int> row_of(S), step_of_l(std::max(S, 1), -1);
+  std::vector<int> step_of_l(std::max(S, 1), -1);
   for (int k = 0; k < n; ++k)
     for (int e = hp.proc_ptr[k]; e < hp.proc_ptr[k + 1]; ++e) {
-      row_of[e] = k;
       step_of_l[hp.proc_lidx[e]] = e;
     }
   auto end_of = [&](int k) { return hp.proc_ptr[k + 1] > hp.proc_ptr[k] ? hp.proc_ptr[k + 1] - 1 : S + k; };
@@ -56,7 +52,8 @@ static bool schedule_tile_factor(const HostPattern& hp, const std::vector<int>& 
     succ[a].push_back(b);
     ++npred[b];
   };
-  std::vector<std::vector<std::pair<int, int>>> upd(S);  // {slot index in the row, the earlier row's step}
+  out->upd.assign(S, {});
+  auto& upd = out->upd;
   std::vector<int> final_by(S);  // the task after which a step's y is final
   for (int k = 0; k < n; ++k) {
     const int p0 = hp.proc_ptr[k], p1 = hp.proc_ptr[k + 1], ni = 1 + hp.init_ptr[k + 1] - hp.init_ptr[k];
@@ -118,11 +115,11 @@ static bool schedule_tile_factor(const HostPattern& hp, const std::vector<int>& 
   std::stable_sort(by_late.begin(), by_late.end(), [&](int a, int b) { return late(a) < late(b); });
   // ---- schedule ----
   const int W = kTfWarps;
+  auto schedule = [&](int look, std::vector<int> npred, HostTileSchedule* result) -> bool {
+  HostTileSchedule& H = *result;
   std::vector<int> tick(N, -1), warp(N, -1), load_tick(n, -1), dep_tick(N, -1), dep_warp(N, -1);
-  struct Op {
-    int tick, task;  // task: step, S + row: init, N + row: load
-  };
-  std::vector<std::vector<Op>> ops(W);
+  auto& ops = H.ops;
+  ops.assign(W, {});
   struct Ready {
     int tail, task, warp;  // warp -1: any
     bool operator<(const Ready& o) const { return tail != o.tail ? tail < o.tail : task > o.task; }
@@ -195,7 +192,9 @@ static bool schedule_tile_factor(const HostPattern& hp, const std::vector<int>& 
     values.push_back({load_tick[k], last_d[k], S + k});
   }
   std::stable_sort(values.begin(), values.end(), [](const Value& a, const Value& b) { return a.from < b.from; });
-  std::vector<int> slot(S + n, 0), spare;
+  std::vector<int> spare;
+  auto& slot = H.slot;
+  slot.assign(S + n, 0);
   std::priority_queue<std::pair<int, int>, std::vector<std::pair<int, int>>, std::greater<std::pair<int, int>>> busy;
   H.slots = 1;
   for (const Value& v : values) {
@@ -213,10 +212,41 @@ static bool schedule_tile_factor(const HostPattern& hp, const std::vector<int>& 
     slot[v.id] = s;
     busy.push({v.to, s});
   }
-  if (H.slots > max_slots) {
-    *why = "the factorization's values in flight do not fit (" + std::to_string(H.slots) + " slots)";
+  return true;
+  };
+  // Rows that start early keep every warp busy and take slots: as early as the
+  // slots of two CTAs per SM allow, else of one.
+  HostTileSchedule best, one;
+  best.slots = INT_MAX;
+  for (int ticks : {kTfDelay + 8, kTfDelay + 2, kTfDelay}) {
+    if (!schedule(kTfTick * ticks, npred, &one)) return false;
+    if (one.slots <= kTfSlots2 || (best.slots > kTfSlots && one.slots < best.slots)) std::swap(best, one);
+    if (best.slots <= kTfSlots2) break;
+  }
+  if (best.slots > kTfSlots) {
+    *why = "the factorization's values in flight do not fit (" + std::to_string(best.slots) + " slots)";
     return false;
   }
+  out->ops.swap(best.ops);
+  out->slot.swap(best.slot);
+  out->slots = best.slots;
+  out->ticks = best.ticks;
+  return true;
+}
+
+bool emit_tile_factor(const HostTileSchedule& sched, const HostPattern& hp, const std::vector<int>& init_slot,
+                      const int* kin, int np, int na, HostTileFactor* out, std::string* why) {
+  HostTileFactor& H = *out;
+  H = HostTileFactor{};
+  H.slots = sched.slots;
+  H.ticks = sched.ticks;
+  const int n = hp.n, S = hp.nnz_l, N = S + n, W = kTfWarps;
+  const auto &ops = sched.ops;
+  const auto &slot = sched.slot;
+  const auto &upd = sched.upd;
+  std::vector<int> row_of(S);
+  for (int k = 0; k < n; ++k)
+    for (int e = hp.proc_ptr[k]; e < hp.proc_ptr[k + 1]; ++e) row_of[e] = k;
   // ---- the lists ----
   H.step_at.assign(S, 0);
   H.row_at.assign(n, 0);
@@ -256,7 +286,7 @@ static bool schedule_tile_factor(const HostPattern& hp, const std::vector<int>& 
         fill4();
       }
     };
-    for (const Op& o : ops[w]) {
+    for (const HostTileSchedule::Op& o : ops[w]) {
       if (o.tick > now) end_ticks(o.tick);
       if (o.task >= N) {
         const int k = o.task - N;
@@ -322,16 +352,6 @@ static bool schedule_tile_factor(const HostPattern& hp, const std::vector<int>& 
     H.prog.insert(H.prog.end(), p.begin(), p.end());
   }
   return true;
-}
-
-// Rows that start early keep every warp busy and take slots: as early as the slots
-// of two CTAs per SM allow, else of one.
-bool build_tile_factor(const HostPattern& hp, const std::vector<int>& init_slot, const int* kin, int np, int na,
-                       HostTileFactor* out, std::string* why) {
-  for (int max_slots : {kTfSlots2, kTfSlots})
-    for (int ticks : {kTfDelay + 8, kTfDelay + 2, kTfDelay})
-      if (schedule_tile_factor(hp, init_slot, kin, np, na, kTfTick * ticks, max_slots, out, why)) return true;
-  return false;
 }
 
 }  // namespace wmpc
