@@ -19,13 +19,15 @@
 // column takes 82 and 99 cycles, beside the items some 140.  HBM is behind
 // (65,536 instances of the 30-step quadrotor class: 3.27 MB per tile and
 // iteration, 26 ms at the measured copy rate).  ADMM of 25 iterations, this form
-// against the streaming form: 2.72 against 5.37 ms for one instance, 40.5
-// against 58.8 ms for 65,536; 1.16 against 2.15 ms for 97 of the 50-step
+// against the streaming form: 2.65 against 5.37 ms for one instance, 39.7
+// against 58.8 ms for 65,536; 1.07 against 2.15 ms for 97 of the 50-step
 // cartpole class.  Measured and left: all items' copies from one producer warp
 // (a bulk copy costs it some 500 cycles with its handshakes: 3.2 ms at one
 // instance, 46.6 ms at 65,536), L loaded two columns ahead (3.4 ms: its
-// registers are the item warps'), 9 or 15 item warps for the 16-row window
-// (3.07, 3.48 ms).
+// registers are the item warps'), 9, 12 or (with spilled registers) 15 item warps
+// for the 16-row window (3.07, 2.72, 3.48 ms); a second CTA per SM for the 50-step
+// cartpole class with rings of little more than an item (16,384 instances, two
+// solves, 9.7 ms against 9.3).
 //
 // Arithmetic is the reference's operation order (warp_backend.py:176-218,
 // solver.py:806-820), every product and sum rounded separately.  Padding
@@ -63,7 +65,7 @@ struct BandArgs {
   BandJob job[kMaxBandJobs];
   int tile_end[kMaxBandJobs];
   int n_jobs, warps, stages;  // item warps, chain stages
-  int vrows, yrows, t4, n_chunks, n_items, chunk_bytes, ring_bytes, spread;
+  int vrows, yrows, t4, n_chunks, n_items, chunk_bytes, ring_bytes;
   int* error;
   unsigned long long wait_limit_ns;
 };
@@ -382,11 +384,14 @@ __device__ __forceinline__ float band_dot(float sum, int units, const int4* rows
 // items never overlap the F items of the phase before.
 // Items belong to a warp for the whole solve: it writes their iterates with
 // ordinary stores and copies them back itself an iteration later.
-// spread: a CTA that has its SM alone runs 16 or 20 warps, every fourth of which
-// (one scheduler's) is the chain, its producer or idle: the chain warp issues
-// without competition.  Else warps 0, 1, the rest.
+// Warps: 0 the chain, 4 its producer (on the same scheduler: 65,536 quadrotor
+// instances 39.7 ms, with warp 1 in its place 41.0), the rest items.  (As many
+// items as the registers allow: with two or three warps left idle so that the
+// chain's scheduler issues for it alone, all cases took 2 to 7 % longer.)
 // kWide: the launch has a class with a 16-row window, whose chain code needs 128
 // registers.
+constexpr int kProducerWarp = 4;
+
 template <bool kTrack, bool kRho, bool kWide>
 __global__ void __launch_bounds__(kWide ? 512 : 640, 1) band_admm_kernel(const __grid_constant__ BandArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -464,8 +469,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 640, 1) band_admm_kernel(const _
     return kTrack && J.check_every > 0 && it > 0 && it % J.check_every == 0 && it < J.max_iter;
   };
 
-  const int role = a.spread ? ((warp & 3) ? 2 : warp >> 2) : warp;  // chain, its producer, items
-  if (role == 0) {
+  if (warp == 0) {
     // ------------------------------ chain ------------------------------
     int stage = 0, have = -1, ordinal = 0;
     uint32_t phase = 0;
@@ -579,7 +583,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 640, 1) band_admm_kernel(const _
       }
     }
     if (!ok && lane == 0) *abort_flag = 1;
-  } else if (role == 1) {
+  } else if (warp == kProducerWarp) {
     // -------------------------- chain producer --------------------------
     uint32_t issued = 0;
     int stage = 0, ordinal = 0, have = -1;
@@ -646,8 +650,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 640, 1) band_admm_kernel(const _
     }
   } else {
     // ------------------------------ items ------------------------------
-    const int iw = a.spread ? (warp >> 2) * 3 + (warp & 3) - 1 : warp - 2;
-    const bool idle = iw >= K || (a.spread && (warp & 3) == 0);
+    const int iw = warp - 1 - (warp > kProducerWarp);
     int have = -1;
     unsigned chunks = 0, phases = 0;  // chain chunks and B phases of the phases gone by
     unsigned chain_seen = 0;          // counter as last read
@@ -657,7 +660,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 640, 1) band_admm_kernel(const _
       if (last >= target) return true;
       return band_poll<2, 100>([&] { return (last = ld_acquire_cta(ctr)) >= target; }, abort_flag, a.wait_limit_ns);
     };
-    for (int g = blockIdx.x; g < total && ok && !idle; g += gridDim.x) {
+    for (int g = blockIdx.x; g < total && ok; g += gridDim.x) {
       const int c = band_job_of(a, g);
       const BandJob& J = a.job[c];
       const BandPlan& bp = J.bp;
@@ -1068,11 +1071,9 @@ int band_run(const BandJobDesc* jobs, int n_jobs, int* error, int num_sms, cudaS
   BandArgs a{};
   int ctas = 1;
   size_t room = (size_t)kMaxSmemBytes;
-  a.spread = 1;
   a.warps = z.warps();
   if (!z.wide && limit >= 2 && total > num_sms && z.bytes(8, 2 * z.item) <= (size_t)(sm_bytes / 2 - reserved)) {
     ctas = 2;
-    a.spread = 0;
     a.warps = 8;
     room = (size_t)(sm_bytes / 2 - reserved);
   }
@@ -1111,7 +1112,7 @@ int band_run(const BandJobDesc* jobs, int n_jobs, int* error, int num_sms, cudaS
                                      (int)cudaSharedmemCarveoutMaxShared));
   const int grid = total < ctas * num_sms ? total : ctas * num_sms;
   profile_mark_begin(s);
-  kernel<<<grid, a.spread ? (a.warps + 2) / 3 * 128 : 32 * (a.warps + 2), smem, s>>>(a);
+  kernel<<<grid, 32 * (a.warps + 2), smem, s>>>(a);
   profile_mark_end(s);
   record_stream_launch(3, ctas, grid, (int)smem);
   WMPC_LAUNCH_CHECK();

@@ -22,8 +22,8 @@
 namespace wmpc {
 
 constexpr int kBandStages = 3;         // chain chunks in flight
-constexpr int kBandWarps = 15;         // item warps of a CTA that has its SM alone
-constexpr int kBandWideWarps = 12;     // the same for a 16-row window, whose chain needs more registers
+constexpr int kBandWarps = 18;         // item warps of a CTA that has its SM alone
+constexpr int kBandWideWarps = 14;     // the same for a 16-row window, whose chain needs more registers
 constexpr int kBandChildren = 2;       // children of a root, at most
 constexpr int kBandUsesPre = 1 << 15;  // item word flag: reads pre-chain values
 
