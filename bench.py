@@ -135,8 +135,8 @@ class ClockSampler:
 def algorithmic_bytes_per_instance(plan, max_iter):
     """Roofline bytes of one persistent solve of one instance (float32).
 
-    factor (factor_stream_kernel): KKT values read + L, D, D^-1 written; each
-    ADMM iteration (admm_stream_kernel): L read twice (forward and backward
+    factor (tile_factor_kernel): KKT values read + L, D, D^-1 written; each
+    ADMM iteration (ADMM kernel): L read twice (forward and backward
     sweep) + D^-1 read.  Index tables are shared by all instances and
     amortised to zero.  Returns (whole solve, factor, one iteration).
     """
@@ -918,8 +918,9 @@ def main():
     # the schedule form, CTAs per SM and grid of the step's streaming launch, as the library ran it
     launch = native.stream_last_launch()
     form = launch["form"] or "plain"
-    # dominant kernel (admm_stream_kernel) and the factorization kernel
-    # (factor_stream_kernel) each timed alone over the timed-region workload
+    kernel = "band_admm_kernel" if form == "band" else "admm_stream_kernel"
+    # dominant kernel (the ADMM kernel of the form) and the factorization kernel
+    # (tile_factor_kernel) each timed alone over the timed-region workload
     # (eager, same inputs; the library's event pair around each launch, on its stream)
     native.profile_begin(native.PROFILE_DOMINANT)
     for _ in range(args.steps):
@@ -932,8 +933,8 @@ def main():
     dom_ms_per_launch = dom_ms / max(dom_n, 1)
     fac_ms_per_launch = fac_ms / max(fac_n, 1)
     per_inst, fac_b, it_b = algorithmic_bytes_per_instance(plan, plan.settings.max_iter)
-    admm_bytes = plan.settings.max_iter * it_b * B  # what admm_stream_kernel alone must move
-    factor_bytes = fac_b * B                         # what factor_stream_kernel alone must move
+    admm_bytes = plan.settings.max_iter * it_b * B  # what the ADMM kernel alone must move
+    factor_bytes = fac_b * B                         # what the factorization alone must move
     peaks = {}
     try:
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as fh:
@@ -946,17 +947,18 @@ def main():
     fac_achieved = factor_bytes / (fac_ms_per_launch * 1e-3) / 1e9 if fac_n else None
     roofline = {
         "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-        "traffic": measured_traffic(args, B, form), "kernel": "admm_stream_kernel", "schedule": form,
+        "traffic": measured_traffic(args, B, "plain" if form == "band" else form, kernel), "kernel": kernel,
+        "schedule": form,
         "ctas_per_sm": launch["ctas_per_sm"], "kernel_ms": dom_ms_per_launch, "launches_timed": dom_n,
         "bytes_per_launch": admm_bytes, "tuned_schedule": schedule, "tune_timings_ms": tune_timings,
         "bytes_rule": f"{plan.settings.max_iter} iterations x 4 (2 nnz(L) + n) per instance",
         "peak_source": peak_source,
         "factor": {
-            "kernel": "factor_stream_kernel", "kernel_ms": fac_ms_per_launch, "launches_timed": fac_n,
+            "kernel": "tile_factor_kernel", "kernel_ms": fac_ms_per_launch, "launches_timed": fac_n,
             "bytes_per_launch": factor_bytes, "bytes_rule": "4 (nnz(KKT) + nnz(L) + 2 n) per instance",
             "achieved": fac_achieved, "peak": peak, "unit": "GB/s",
             "frac": (fac_achieved / peak) if fac_achieved else None,
-            "traffic": measured_traffic(args, B, "plain", "factor_stream_kernel"),
+            "traffic": measured_traffic(args, B, "plain", "tile_factor_kernel"),
         },
     }
 

@@ -16,11 +16,11 @@
 // alike.  Per column the forward sweep's updates of the window are independent
 // of one another, the backward sweep's sum is a serial chain of additions (the
 // reference's order starts with the row solved last): alone on an SM a 16-row
-// column takes 82 and 99 cycles, beside the items some 140.  HBM is behind
-// (65,536 instances of the 30-step quadrotor class: 3.27 MB per tile and
-// iteration, 26 ms at the measured copy rate).  ADMM of 25 iterations, this form
-// against the streaming form: 2.65 against 5.37 ms for one instance, 39.7
-// against 58.8 ms for 65,536; 1.07 against 2.15 ms for 97 of the 50-step
+// column takes 82 and 99 cycles, a third of the launch's time per column.  HBM is
+// behind (0.66 of the copy rate with a tile on every SM; 65,536 instances of the
+// 30-step quadrotor class: 3.27 MB per tile and iteration, 26 ms at the copy rate).
+// ADMM of 25 iterations, this form against the streaming form: 2.62 against 5.37
+// ms for one instance, 39.7 against 58.8 ms for 65,536; 1.06 against 2.15 ms for 97 of the 50-step
 // cartpole class.  Measured and left: all items' copies from one producer warp
 // (a bulk copy costs it some 500 cycles with its handshakes: 3.2 ms at one
 // instance, 46.6 ms at 65,536), L loaded two columns ahead (3.4 ms: its
