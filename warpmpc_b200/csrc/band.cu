@@ -19,8 +19,8 @@
 // column takes 82 and 99 cycles, a third of the launch's time per column.  HBM is
 // behind (0.66 of the copy rate with a tile on every SM; 65,536 instances of the
 // 30-step quadrotor class: 3.27 MB per tile and iteration, 26 ms at the copy rate).
-// ADMM of 25 iterations, this form against the streaming form: 2.62 against 5.37
-// ms for one instance, 39.7 against 58.8 ms for 65,536; 1.06 against 2.15 ms for 97 of the 50-step
+// ADMM of 25 iterations, this form against the streaming form: 2.68 against 5.37
+// ms for one instance, 40.0 against 58.8 ms for 65,536; 1.07 against 2.15 ms for 97 of the 50-step
 // cartpole class.  Measured and left: all items' copies from one producer warp
 // (a bulk copy costs it some 500 cycles with its handshakes: 3.2 ms at one
 // instance, 46.6 ms at 65,536), L loaded two columns ahead (3.4 ms: its
@@ -744,6 +744,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 640, 1) band_admm_kernel(const _
           rec = mine + head;
         };
         auto release = [&]() {
+          if (per_it <= 4) __threadfence();  // (its next copy may follow at once; else a phase's fence lies between)
           __syncwarp();
           head += size;
           if (--flying == 0) {

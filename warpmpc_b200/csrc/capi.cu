@@ -383,13 +383,13 @@ bool band_wanted() {
 // may go on (some 2.5 us per column and iteration, against 0.2 per chain row):
 // it loses where the chain is not much longer.  Where the chain is 10 to 20
 // times as long it wins only up to one tile per SM: with more, the streaming
-// form shares an SM between two or three tiles.  ADMM of 25 iterations, us, band
+// form shares an SM between two tiles.  ADMM of 25 iterations, us, band
 // against streaming form, at 2000 / 9000 / 60,000 instances:
-//   20-step 6-state class (T 79, 12)     1059 / 1599 / 10408 against  937 / 1135 / 8172
-//   10-step quadrotor class (T 121, 7)   1323 / 2671 / 17380 against 1800 / 2401 / 16562
-//   40-step 6-state class (T 159, 12)    1555 / 3109 / 20639 against 1830 / 2597 / 17764
-//   20-step cartpole class (T 83, 4)      618 / 1062 /  6908 against  898 / 1059 / 8041
-//   20-step quadrotor class (T 241, 7)   2064 / 4160 / 26825 against 3506 / 5056 / 35956
+//   20-step small class (T 79, 12)       1008 / 1483 /  9898 against  932 / 1137 /  8154
+//   10-step quadrotor class (T 121, 7)   1269 / 2557 / 16459 against 1789 / 2406 / 16627
+//   40-step small class (T 159, 12)      1500 / 3003 / 19409 against 1819 / 2599 / 17822
+//   20-step cartpole class (T 83, 4)      570 /  988 /  6654 against  892 / 1043 /  8132
+//   20-step quadrotor class (T 241, 7)   2085 / 4344 / 27593 against 3489 / 5069 / 36004
 int band_tile_limit(const BandPlan& bp, int num_sms) {
   if (getenv("WMPC_STREAM_BAND")) return INT_MAX;  // asked for
   if (bp.T >= 20 * bp.n_pre) return INT_MAX;

@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(32 * kResParts * kSplit) residual_kernel(
 // Four threads per part up to two tiles per SM, where the loop's latency is what
 // the kernel takes (us: one 30-step quadrotor instance 173 to 79, 1000 of them 396
 // to 135); with more tiles one thread per part fills the SMs (65,536 instances of
-// the 10-step 6-state class 165, split 231).
+// the 10-step small class (4 states) 165, split 231).
 void launch_residual(const Osqp& o, const float* pT, long long ldp, int sbp, const float* aT, long long lda, int sba,
                      const State& st, const float* qT, float* prim, float* dual, float* obj, int* status, int batch,
                      const int* status_in, const int* abort_word, float eps_abs, float eps_rel, int num_sms,

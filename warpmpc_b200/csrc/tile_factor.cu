@@ -49,7 +49,7 @@ struct TileFactorOut {
 // class, issued at 0.39 per cycle and scheduler), not memory.  One tile of that
 // class: 0.58 ms, where one warp per tile with L re-read from memory took 4.97
 // ms; 65,536 instances 5.16 ms against 8.17; 97 of the 50-step cartpole class
-// 0.29 against 1.64; 65,536 of the 10-step 6-state class 0.49 against 0.53; 5000
+// 0.29 against 1.64; 65,536 of the 10-step small class (4 states) 0.49 against 0.53; 5000
 // of the 40-step nonlinear quadrotor QP 2.03 against 7.73.
 template <bool kPlanes>
 __global__ void __launch_bounds__(32 * kTfWarps, 2)
