@@ -364,7 +364,9 @@ int wmpc_band_tables_host(const wmpc_pattern_desc* desc, const float* rho, const
 /* The tile factorization's lists for a pattern whose inputs are the KKT values
  * themselves and whose results go to L's entries in order and D^-1 by row
  * (warpmpc_b200/csrc/tile_factor.cuh), built on the host: no device needed.
- * out: [warps, delay, slots, ticks, words] warp_off[warps] prog[words]. */
+ * out: [warps, delay, slots, ticks, words] piece_wait[delay + 1] warp_off[warps]
+ * prog[words]; piece_wait: copy groups that may be under way when a list goes on at
+ * a piece asked for that many ticks earlier (-1: not even this tick's copies). */
 int wmpc_tile_factor_host(const wmpc_pattern_desc* desc, int32_t* out, int64_t out_capacity, int64_t* out_words);
 
 /* Profiling (no counterpart in the reference, which times with wall

@@ -606,6 +606,7 @@ int wmpc_tile_factor_host(const wmpc_pattern_desc* desc, int32_t* out, int64_t o
     return fail(WMPC_ERR_UNSUPPORTED, "%s", why.c_str());
   place_tile_factor(boff.data(), boff.data(), doff.data(), &t);
   std::vector<int> w{kTfWarps, kTfDelay, t.slots, t.ticks, (int)t.prog.size()};
+  for (int ago = 0; ago <= kTfDelay; ++ago) w.push_back(tf_piece_wait(ago));
   w.insert(w.end(), t.warp_off.begin(), t.warp_off.end());
   w.insert(w.end(), t.prog.begin(), t.prog.end());
   *out_words = static_cast<int64_t>(w.size());

@@ -50,6 +50,14 @@ constexpr int kTfTick = 400;    // a warp's work per tick, in cycles as the sche
 constexpr int kTfSlots = 1536;  // slots, at most (0 is a dummy): one CTA per SM
 constexpr int kTfSlots2 = 624;  // for two
 
+// A list goes on at a piece that was asked for `ago` ticks earlier.  Copies become
+// a group when their tick ends: how many groups may still be under way, or -1 where
+// the copies of this tick, no group yet, have to land as well (rows of a few hundred
+// inputs fill several pieces within a tick).
+__host__ __device__ constexpr int tf_piece_wait(int ago) {
+  return ago >= kTfDelay ? kTfDelay - 1 : ago > 0 ? 0 : -1;
+}
+
 struct TileFactor {
   const int4* prog = nullptr;  // null: not available
   const int* warp_off = nullptr;  // [kTfWarps] first word of each list

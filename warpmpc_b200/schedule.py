@@ -97,7 +97,9 @@ def tile_factor_lists(qp) -> dict | None:
     buf = np.empty(words.value, dtype=np.int32)
     native.check(lib.wmpc_tile_factor_host(ctypes.byref(desc), native.ptr_i32(buf), buf.size, ctypes.byref(words)))
     out = {k: int(v) for k, v in zip(("warps", "delay", "slots", "ticks", "words"), buf)}
-    out["warp_off"], out["prog"] = buf[5 : 5 + out["warps"]].copy(), buf[5 + out["warps"] :].reshape(-1, 4).copy()
+    waits, lists = np.split(buf[5:], [out["delay"] + 1])
+    out["piece_wait"] = waits.copy()
+    out["warp_off"], out["prog"] = lists[: out["warps"]].copy(), lists[out["warps"] :].reshape(-1, 4).copy()
     return out
 
 
