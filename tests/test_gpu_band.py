@@ -187,3 +187,51 @@ def test_given_factorization(cuda_device, monkeypatch, band, cls, batch, shared)
         zero = (status & native.STATUS_ZERO_PIVOT) != 0
         assert torch.equal(status & ~native.STATUS_ZERO_PIVOT, comp.engine.last_status)
         assert zero.nonzero().flatten().tolist() == ([17] if batch > 1 and not shared else [])
+
+
+def _sum_qp(n, k, batch, seed):
+    """``n`` variables with bounds, one constraint over the first ``k``: a chain of a
+    few rows, most subtrees (with k < n) without an entry in it."""
+    import scipy.sparse as sp
+
+    from warpmpc_b200.jax_osqp.planning import build_osqp_plan
+
+    rng = np.random.default_rng(seed)
+    a = sp.vstack([sp.csr_matrix((np.arange(n) < k).astype(float)[None]), sp.identity(n)]).tocsc()
+    bound = np.full(n + 1, 0.5)
+    plan = build_osqp_plan(sp.identity(n, format="csc"), a, -bound, bound,
+                           OSQPSettings(**{**problems.DEFAULT_SETTINGS, "max_iter": 60}))
+    f = lambda lo, hi, w: rng.uniform(lo, hi, (batch, w)).astype(np.float32)  # noqa: E731
+    lim = np.tile(bound.astype(np.float32), (batch, 1))
+    return plan, (f(0.5, 2.0, plan.nnz_p), f(0.2, 1.0, plan.nnz_a), f(-2.0, 2.0, n), -lim, lim)
+
+
+def _short_chain(name, batch):
+    if name.startswith("sum"):
+        return _sum_qp(60, int(name[3:]), batch, seed=8)
+    nu, box, horizon = (2, 1.0, int(name[5:])) if name.startswith("small") else (1, 10.0, int(name[8:]))
+    b = problems.make_batch(problems.MPCClass(name, 4, nu, horizon, 5.0, box, 2.0, "small"), batch, seed=3)
+    plan = problems.make_plan(b, OSQPSettings(**{**problems.DEFAULT_SETTINGS, "max_iter": 60}))
+    return plan, (b.p_values, b.a_values, b.q, b.l, b.u)
+
+
+@pytest.mark.parametrize("batch", [40, 9500])
+@pytest.mark.parametrize("name", ["small1", "small2", "cartpole1", "cartpole2", "sum60", "sum5"])
+def test_band_form_termination_checks_of_short_chains(cuda_device, monkeypatch, name, batch):
+    """Fewer chain rows than item warps: warps without a row write their maxima in
+    another phase than the rest, and every warp has to come to the same decision."""
+    plan, qp = _short_chain(name, batch)
+    args = _dev(*qp)
+    band, plain = _compile(monkeypatch, plan, 1), _compile(monkeypatch, plan, 0)
+    for check in (1, 5):
+        for warm in (None, tuple(_dev(*_warm(plan, batch, 8)))):
+            got = band.engine.solve(*args, warm=warm, check_termination=check)
+            assert native.stream_last_launch()["form"] == "band"
+            want = plain.engine.solve(*args, warm=warm, check_termination=check)
+            assert native.stream_last_launch()["form"] != "band"
+            for g, w in zip(got, want):
+                np.testing.assert_array_equal(g.cpu().numpy(), w.cpu().numpy())
+            iters = band.engine.last_iters.cpu().numpy()
+            np.testing.assert_array_equal(iters, plain.engine.last_iters.cpu().numpy())
+            np.testing.assert_array_equal(band.engine.last_status.cpu().numpy(), plain.engine.last_status.cpu().numpy())
+            assert iters.min() < 60

@@ -65,7 +65,7 @@ struct BandArgs {
   BandJob job[kMaxBandJobs];
   int tile_end[kMaxBandJobs];
   int n_jobs, warps, stages;  // item warps, chain stages
-  int vrows, yrows, t4, n_chunks, n_items, chunk_bytes, ring_bytes;
+  int vrows, yrows, t4, n_chunks, n_items, chunk_bytes, ring_bytes, maxima_sets;
   int* error;
   unsigned long long wait_limit_ns;
 };
@@ -404,8 +404,8 @@ __global__ void __launch_bounds__(kWide ? 512 : 640, 1) band_admm_kernel(const _
   int4* chunkw = reinterpret_cast<int4*>(reinterpret_cast<unsigned char*>(colw) + (a.t4 * 4 + 15) / 16 * 16);
   int2* pchunk = reinterpret_cast<int2*>(chunkw + a.n_chunks);  // the chain producer's {offset, bytes | columns << 24}
   unsigned* itemw = reinterpret_cast<unsigned*>(pchunk + a.n_chunks);
-  float* maxima = reinterpret_cast<float*>(itemw + (K * a.n_items + 1) / 2 * 2);  // [K][2][32]
-  uint64_t* cfull = reinterpret_cast<uint64_t*>(maxima + K * 64);
+  float* maxima = reinterpret_cast<float*>(itemw + (K * a.n_items + 1) / 2 * 2);  // [maxima_sets][K][2][32]
+  uint64_t* cfull = reinterpret_cast<uint64_t*>(maxima + a.maxima_sets * K * 64);
   uint64_t* cempty = cfull + a.stages;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(cempty + a.stages);
   unsigned* chain_done = reinterpret_cast<unsigned*>(cempty + a.stages) + 1;
@@ -453,11 +453,13 @@ __global__ void __launch_bounds__(kWide ? 512 : 640, 1) band_admm_kernel(const _
   // change and primal residual over the iteration, over all item warps
   bool frozen = false;
   int frozen_at = 0;
+  auto maxima_of = [&](int it) { return maxima + (a.maxima_sets > 1 ? (it & 1) * K * 64 : 0); };
   auto decide = [&](const BandJob& J, int it) -> bool {
+    const float* all = maxima_of(it);
     float chg = 0.0f, pres = 0.0f;
     for (int w = 0; w < K; ++w) {
-      chg = fmaxf(chg, maxima[w * 64 + lane]);
-      pres = fmaxf(pres, maxima[w * 64 + 32 + lane]);
+      chg = fmaxf(chg, all[w * 64 + lane]);
+      pres = fmaxf(pres, all[w * 64 + 32 + lane]);
     }
     if (!frozen && chg <= J.chg_eps && pres <= J.chg_eps) {
       frozen = true;
@@ -830,9 +832,12 @@ __global__ void __launch_bounds__(kWide ? 512 : 640, 1) band_admm_kernel(const _
           if (!ok) break;
           if (it > 0) chunks += (unsigned)bp.n_chunks;
           ++phases;
-          if (kTrack && mf == 0) {
-            maxima[iw * 64 + lane] = u.chg;
-            maxima[iw * 64 + 32 + lane] = u.pres;
+          // (not before the first iteration: after a tile that stopped early a warp may
+          // still be reading that set)
+          if (kTrack && mf == 0 && it > 0) {
+            float* m = maxima_of(it) + iw * 64;
+            m[lane] = u.chg;
+            m[32 + lane] = u.pres;
           }
           publish();
           if (lane == 0) atomicAdd(b_done, 1u);
@@ -871,8 +876,9 @@ __global__ void __launch_bounds__(kWide ? 512 : 640, 1) band_admm_kernel(const _
                 *vr = acc;
             }
             if (kTrack && j == mf - 1) {  // published with the phase's last row
-              maxima[iw * 64 + lane] = u.chg;
-              maxima[iw * 64 + 32 + lane] = u.pres;
+              float* m = maxima_of(it) + iw * 64;
+              m[lane] = u.chg;
+              m[32 + lane] = u.pres;
             }
             release();
             if (j >= n_pre) {
@@ -1010,7 +1016,7 @@ namespace {
 
 // A launch's sizes over its classes, and its shared memory.
 struct BandSizes {
-  int vrows = 0, yrows = 0, t4 = 0, n_chunks = 0, chunk = 0, item = 0;
+  int vrows = 0, yrows = 0, t4 = 0, n_chunks = 0, chunk = 0, item = 0, rows = 1 << 30;  // rows: the shortest chain's
   bool wide = false;
   std::vector<const BandPlan*> plans;
   void add(const BandPlan& bp) {
@@ -1020,6 +1026,7 @@ struct BandSizes {
     n_chunks = std::max(n_chunks, bp.n_chunks);
     chunk = std::max(chunk, bp.chunk_bytes);
     item = std::max(item, bp.item_bytes);
+    rows = std::min(rows, bp.T);
     wide = wide || bp.units > 2;
     plans.push_back(&bp);
   }
@@ -1030,7 +1037,8 @@ struct BandSizes {
     return v;
   }
   size_t bytes(int w, int ring) const {
-    return band_smem_bytes(vrows, yrows, t4, n_chunks, items(w), chunk, ring, w, kBandStages);
+    return band_smem_bytes(vrows, yrows, t4, n_chunks, items(w), chunk, ring, w, kBandStages,
+                           band_maxima_sets(rows, w));
   }
 };
 
@@ -1087,6 +1095,7 @@ int band_run(const BandJobDesc* jobs, int n_jobs, int* error, int num_sms, cudaS
   a.n_chunks = z.n_chunks;
   a.n_items = z.items(a.warps);
   a.chunk_bytes = z.chunk;
+  a.maxima_sets = band_maxima_sets(z.rows, a.warps);
   a.ring_bytes = std::min(16384, z.item + (int)((room - least) / a.warps) / 128 * 128);
   const size_t smem = z.bytes(a.warps, a.ring_bytes);
   int end = 0;

@@ -123,14 +123,21 @@ int band_state_out(const BandPlan& bp, const BandWork& w, float* x, float* z, fl
 // whether one launch can hold these classes
 bool band_fits(const BandPlan* const* plans, int n);
 int band_run(const BandJobDesc* jobs, int n_jobs, int* error, int num_sms, cudaStream_t s);
-// bytes of shared memory a CTA of `warps` item warps, `stages` chain stages and
-// `groups` group stages takes
 // items of an iteration in item warp 0's list (the longest)
 inline int band_items(int n_pre, int nb, int T, int warps) {
   return 2 * n_pre + (nb + warps - 1) / warps + (T + warps - 1) / warps;
 }
 
+// Sets of per-warp maxima a CTA needs.  A warp with a chain row writes its maxima in
+// the F phase, once every warp has read those of the iteration before.  One without
+// (a chain of fewer rows than item warps) writes them at the end of its B phase,
+// which waits for no other item warp's decision: two sets, by iteration parity, put
+// an F phase between a set's last read and its next write.
+inline int band_maxima_sets(int T, int warps) { return T < warps ? 2 : 1; }
+
+// bytes of shared memory a CTA of `warps` item warps, `stages` chain stages and
+// `maxima_sets` sets of maxima takes
 size_t band_smem_bytes(int vrows, int yrows, int t4, int n_chunks, int n_items, int chunk_bytes, int ring_bytes,
-                       int warps, int stages);
+                       int warps, int stages, int maxima_sets);
 
 }  // namespace wmpc

@@ -8,11 +8,11 @@
 namespace wmpc {
 
 size_t band_smem_bytes(int vrows, int yrows, int t4, int n_chunks, int n_items, int chunk_bytes, int ring_bytes,
-                       int warps, int stages) {
+                       int warps, int stages, int maxima_sets) {
   size_t b = (size_t)(vrows + yrows) * 128 + (size_t)stages * chunk_bytes + (size_t)warps * ring_bytes;
   b += (size_t)((t4 * 4 + 15) / 16) * 16 + (size_t)n_chunks * 24;  // column words, chunk descriptors (chain, producer)
   b += (size_t)((warps * n_items + 1) / 2) * 8;                    // item words
-  b += (size_t)warps * 256;                                        // iterate changes and residuals per warp
+  b += (size_t)maxima_sets * warps * 256;                          // iterate changes and residuals per warp
   b += (size_t)stages * (16 + 4) + 64 + (size_t)warps * 4;         // barriers, tags, counters
   return (b + 127) / 128 * 128;
 }
@@ -381,7 +381,8 @@ bool build_band_tables(const HostPattern& hp, const float* rho, const float* rho
   H.blen = off;
   const int warps = H.units > 2 ? kBandWideWarps : kBandWarps;
   if (band_smem_bytes(band_vrows(T4, H.units, n_pre), H.n_yr + 1, T4, H.n_chunks, band_items(n_pre, H.nb, T, warps),
-                      H.chunk_bytes, H.item_bytes, warps, kBandStages) > (size_t)kMaxSmemBytes) {
+                      H.chunk_bytes, H.item_bytes, warps, kBandStages, band_maxima_sets(T, warps)) >
+      (size_t)kMaxSmemBytes) {
     *why = "band work vectors do not fit in shared memory";
     return false;
   }
