@@ -235,3 +235,17 @@ def test_band_form_termination_checks_of_short_chains(cuda_device, monkeypatch, 
             np.testing.assert_array_equal(iters, plain.engine.last_iters.cpu().numpy())
             np.testing.assert_array_equal(band.engine.last_status.cpu().numpy(), plain.engine.last_status.cpu().numpy())
             assert iters.min() < 60
+
+
+@pytest.mark.parametrize("k,batch", [(5, 1), (5, 9500), (60, 33)])
+def test_band_form_decoupled_variables(cuda_device, monkeypatch, k, batch):
+    """Subtrees that read no chain row: they read the zero row, no sooner than it is written."""
+    from oracle.cpu_baseline import CpuOSQP
+
+    plan, qp = _sum_qp(60, k, batch, seed=5)
+    comp = _compile(monkeypatch, plan, 1)
+    for iters in (1, 2, 7):
+        got = comp.engine.solve(*_dev(*qp), max_iter=iters)
+        assert native.stream_last_launch()["form"] == "band"
+        for g, r in zip(got[:3], CpuOSQP(plan).solve(*qp, max_iter=iters)[:3]):
+            np.testing.assert_array_equal(g.cpu().numpy(), r)

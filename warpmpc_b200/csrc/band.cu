@@ -377,7 +377,7 @@ __device__ __forceinline__ float band_dot(float sum, int units, const int4* rows
 // sweeps finished), b_done (B phases finished, once per item warp), f_done
 // (chain rows finished in F phases, per item warp), pre_b / pre_f (phases in
 // which the pre-chain is solved / its right-hand sides are formed).  Waits: a
-// B item for the chunks it reads; an F item for every B item (b_done) and the
+// B item for the chunks it reads, at least one; an F item for every B item (b_done) and the
 // whole backward sweep; items that read pre-chain values for item warp 0,
 // which does them first; a forward chunk for the F items of its rows and of
 // the rows it adds to.  A backward sweep follows the whole forward sweep, so B

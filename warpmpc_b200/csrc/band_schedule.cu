@@ -241,8 +241,11 @@ bool build_band_tables(const HostPattern& hp, const float* rho, const float* rho
   for (int c = 0; c < n; ++c)
     if (!rest[c] && !child[c]) {
       sub_of[c] = static_cast<int>(subs.size());
-      // (after the pre-chain, where it is read: its own chunks and some slack)
-      subs.push_back(Sub{c, uses_pre(c) ? std::min(H.n_chunks, std::max(need_of(c), pre_need + 1)) : need_of(c), {}});
+      // (after the pre-chain, where it is read: its own chunks and some slack; one chunk
+      // where it reads no chain row: the zero row of its padding and of its children's
+      // slots is written in the first F phase, which the chain waits for)
+      subs.push_back(
+          Sub{c, uses_pre(c) ? std::min(H.n_chunks, std::max(need_of(c), pre_need + 1)) : std::max(need_of(c), 1), {}});
     }
   for (int c = 0; c < n; ++c)
     if (child[c]) subs[sub_of[li[lp[c]]]].child.push_back(c);
