@@ -377,8 +377,8 @@ __device__ __forceinline__ float band_dot(float sum, int units, const int4* rows
 // sweeps finished), b_done (B phases finished, once per item warp), f_done
 // (chain rows finished in F phases, per item warp), pre_b / pre_f (phases in
 // which the pre-chain is solved / its right-hand sides are formed).  Waits: a
-// B item for the chunks it reads, at least one; an F item for every B item (b_done) and the
-// whole backward sweep; items that read pre-chain values for item warp 0,
+// B item for the chunks it reads, at least one; an F item for every B item (b_done)
+// and the whole backward sweep; items that read pre-chain values for item warp 0,
 // which does them first; a forward chunk for the F items of its rows and of
 // the rows it adds to.  A backward sweep follows the whole forward sweep, so B
 // items never overlap the F items of the phase before.
@@ -902,7 +902,10 @@ __global__ void __launch_bounds__(kWide ? 512 : 640, 1) band_admm_kernel(const _
           next_phase(bp.T);
         }
       }
-      cp_async_wait_group<0>();  // (a tile that stopped early has copies in flight)
+      // A tile that stopped early has copies in flight: every lane's have landed before
+      // any lane's for the next tile go to the same bytes.
+      cp_async_wait_group<0>();
+      __syncwarp();
       if (iw == 0 && J.iters && tile * 32 + lane < J.batch) J.iters[tile * 32 + lane] = frozen ? frozen_at : it_run;
     }
     if (!ok && lane == 0) *abort_flag = 1;
