@@ -361,6 +361,10 @@ int wmpc_stream_schedule_host(const wmpc_pattern_desc* desc, const float* rho, c
 int wmpc_band_tables_host(const wmpc_pattern_desc* desc, const float* rho, const float* rhoinv, int32_t n_primal,
                           int32_t* out, int64_t out_capacity, int64_t* out_words);
 
+/* 1 where a band-form item warp with mb and mf items in an iteration's two phases
+ * fences each item's stores by itself (0: the phases' own fences suffice). */
+int wmpc_band_item_fence_host(int32_t mb, int32_t mf);
+
 /* The tile factorization's lists for a pattern whose inputs are the KKT values
  * themselves and whose results go to L's entries in order and D^-1 by row
  * (warpmpc_b200/csrc/tile_factor.cuh), built on the host: no device needed.

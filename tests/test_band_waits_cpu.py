@@ -11,7 +11,7 @@ import scipy.sparse as sp
 
 from oracle import osqp_ref
 from test_band_cpu import replay
-from warpmpc_b200 import problems
+from warpmpc_b200 import native, problems
 from warpmpc_b200.jax_osqp import OSQPSettings
 from warpmpc_b200.jax_osqp.planning import build_osqp_plan
 from warpmpc_b200.schedule import band_tables
@@ -59,3 +59,41 @@ def test_band_replay_of_decoupled_variables(k):
     ref = osqp_ref.solve(plan, b.p_values, b.a_values, b.q, b.l, b.u, max_iter=3)
     for g, r in zip(got, ref[:3]):
         np.testing.assert_array_equal(g, r)
+
+
+def unfenced(mb, mf, fence, ahead=4, iters=4):
+    """Items of a warp (mb, then mf per iteration) whose iterate is copied back with
+    neither the end of a phase nor a fence of its own since it was stored.  Copies run
+    ahead as far as their number allows (a full ring only delays them)."""
+    per_it, bad = mb + mf, set()
+    flying, next_pos, clean = 0, 0, {}  # clean: item: its last store is fenced
+
+    def fill():
+        nonlocal flying, next_pos
+        while flying < min(ahead, per_it) and next_pos < iters * per_it:
+            item = next_pos % per_it
+            if not clean.get(item, True):
+                bad.add(item)
+            flying, next_pos = flying + 1, next_pos + 1
+
+    fill()
+    for it in range(iters):
+        for item in range(per_it):
+            clean[item] = fence
+            flying -= 1
+            fill()
+            if item in (mb - 1, per_it - 1):
+                clean = dict.fromkeys(clean, True)
+    return bad
+
+
+@pytest.mark.parametrize("mb", range(9))
+def test_items_are_fenced_before_they_are_copied_back(mb):
+    for mf in range(9):
+        if mb + mf:
+            assert not unfenced(mb, mf, bool(native.lib().wmpc_band_item_fence_host(mb, mf))), mf
+
+
+def test_item_fences_are_left_out_where_phases_are_long():
+    assert not native.lib().wmpc_band_item_fence_host(4, 4) and not unfenced(4, 4, False)
+    assert unfenced(3, 4, False) and unfenced(4, 3, False) and unfenced(3, 3, False)

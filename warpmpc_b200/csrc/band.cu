@@ -698,7 +698,8 @@ __global__ void __launch_bounds__(kWide ? 512 : 640, 1) band_admm_kernel(const _
           __syncwarp();
           have = c;
         }
-        const int depth = per_it < 4 ? per_it : 4;
+        const int depth = per_it < kBandAhead ? per_it : kBandAhead;
+        const bool fence = band_item_fence(mb, mf);
         int next_i = 0, next_it = 0;                // the next one to copy
         int head = 0, tail = 0, flying = 0, size = 0;  // the oldest one and its size, the end of the newest, how many
         bool wrapped = false;                       // the newest lies before the oldest
@@ -732,6 +733,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 640, 1) band_admm_kernel(const _
           }
         };
         fill();
+        static_assert(kBandAhead == 4, "take() counts copies in flight up to four");
         auto take = [&](int i) {
           size = (int)(words[i] >> 22) * 128;
           if (head + size > a.ring_bytes) {
@@ -746,7 +748,7 @@ __global__ void __launch_bounds__(kWide ? 512 : 640, 1) band_admm_kernel(const _
           rec = mine + head;
         };
         auto release = [&]() {
-          if (per_it <= 4) __threadfence();  // (its next copy may follow at once; else a phase's fence lies between)
+          if (fence) __threadfence_block();  // (as publish() below)
           __syncwarp();
           head += size;
           if (--flying == 0) {

@@ -128,6 +128,14 @@ inline int band_items(int n_pre, int nb, int T, int warps) {
   return 2 * n_pre + (nb + warps - 1) / warps + (T + warps - 1) / warps;
 }
 
+// An item warp's copies ahead.  An item's copy for the next iteration starts when the
+// item kBandAhead places before it in the warp's list (B items, then F items) is
+// released.  Its iterate was stored a few items before; where the warp has at least
+// kBandAhead items in each phase the end of a phase, with its fence, lies between.
+// Else every item has a fence of its own.
+constexpr int kBandAhead = 4;
+__host__ __device__ constexpr bool band_item_fence(int mb, int mf) { return mb < kBandAhead || mf < kBandAhead; }
+
 // Sets of per-warp maxima a CTA needs.  A warp with a chain row writes its maxima in
 // the F phase, once every warp has read those of the iteration before.  One without
 // (a chain of fewer rows than item warps) writes them at the end of its B phase,

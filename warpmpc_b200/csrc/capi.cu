@@ -565,6 +565,8 @@ int wmpc_band_tables_host(const wmpc_pattern_desc* desc, const float* rho, const
   return WMPC_OK;
 }
 
+int wmpc_band_item_fence_host(int32_t mb, int32_t mf) { return band_item_fence(mb, mf) ? 1 : 0; }
+
 int wmpc_tile_factor_host(const wmpc_pattern_desc* desc, int32_t* out, int64_t out_capacity, int64_t* out_words) {
   if (!desc || !out_words) return fail(WMPC_ERR_INVALID_ARGUMENT, "null argument");
   const int n = desc->n, nnz_l = desc->nnz_l;

@@ -268,6 +268,7 @@ SIGNATURES = {
                                               ctypes.POINTER(ctypes.c_int64)]),
     "wmpc_tile_factor_host": (ctypes.c_int, [ctypes.POINTER(PatternDesc), _i32p, ctypes.c_int64,
                                              ctypes.POINTER(ctypes.c_int64)]),
+    "wmpc_band_item_fence_host": (ctypes.c_int, [ctypes.c_int32, ctypes.c_int32]),
     "wmpc_band_tables_host": (
         ctypes.c_int,
         [ctypes.POINTER(PatternDesc), _f32p, _f32p, ctypes.c_int32, _i32p, ctypes.c_int64,
