@@ -1062,6 +1062,12 @@ __global__ void __launch_bounds__(128, 1) admm_stream_kernel(const __grid_consta
             if (issued_s >= (uint32_t)a.sstages &&
                 !mbar_wait_bounded(sempty + sr.stage, sr.phase ^ 1u, abort_flag, a.wait_limit_ns))
               return false;
+            // the records this chunk's last release wrote (a pass ago).  In a pattern of
+            // fewer chunks than stages a free stage says nothing of that release.
+            if (kind == kItemBwd && sp.n_chunks < a.sstages &&
+                !wait_counter_bounded(rel_done, issued_l - (uint32_t)(sp.n_chunks + sp.n_fchunks), abort_flag,
+                                      a.wait_limit_ns))
+              return false;
             unsigned char* ss = sring + (size_t)sr.stage * a.sbytes;
             const uint32_t nrel = (uint32_t)d.nrel, np = (uint32_t)d.nprim, nc = nrel - np;
             // per region (iterates at 0, parameters at pres_off / 2): the primal
