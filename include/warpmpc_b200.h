@@ -224,7 +224,10 @@ typedef struct wmpc_osqp_batch {
 
 /* Device workspace bytes for `batch` instances.  mode: WMPC_OSQP_PLAIN or
  * WMPC_OSQP_PERSISTENT; external_factor: 1 when the caller passes lx/dinv
- * (solve_with_factor), 0 when the call factors. */
+ * (solve_with_factor), 0 when the call factors.  A persistent solve with a given
+ * factorization copies it into its streams, once per instance; external_factor 2
+ * gives the least such a solve runs in (no copies; several times slower for fixed
+ * iterations, and all that one with check_termination uses). */
 size_t wmpc_osqp_workspace_bytes(const wmpc_osqp* osqp, int32_t batch, int32_t mode, int32_t external_factor);
 
 /* Which streaming schedule the problem carries (no reference counterpart: the

@@ -249,3 +249,45 @@ def test_band_form_decoupled_variables(cuda_device, monkeypatch, k, batch):
         assert native.stream_last_launch()["form"] == "band"
         for g, r in zip(got[:3], CpuOSQP(plan).solve(*qp, max_iter=iters)[:3]):
             np.testing.assert_array_equal(g.cpu().numpy(), r)
+
+
+def test_given_factorization_in_less_memory(cuda_device, monkeypatch):
+    """A given factorization is copied per instance where the memory for it is there;
+    else, and in a checked solve, the workspace is the small one and the iterates
+    are the same."""
+    import torch
+
+    from warpmpc_b200.jax_osqp import solver
+
+    batch = 2500
+    b = problems.make_batch(problems.CARTPOLE, batch, seed=12)
+    plan = problems.make_plan(b)
+    comp = compile_osqp(plan, np.float32, qdldl_backend="cuda", transpose_work=True)
+    engine = comp.engine
+    args = _dev(b.p_values[:1], b.a_values[:1], b.q, b.l, b.u)
+    factor = comp.factor(args[0], args[1])
+    least, room = engine.factor_workspace_bytes(batch), 1 << 60
+    asked = []
+
+    def allocate(nbytes, device):
+        asked.append(nbytes)
+        if nbytes > room:
+            raise torch.OutOfMemoryError("no room for the copies")
+        return torch.empty(int(nbytes), dtype=torch.uint8, device=device), int(nbytes)
+
+    monkeypatch.setattr(solver, "_workspace", allocate)
+    want = engine.solve(*args, factor=factor)
+    assert len(asked) == 1 and asked[0] > 2 * least
+    room = least
+    got = [engine.solve(*args, factor=factor)]
+    assert asked[1:] == [asked[0], least]
+    got.append(engine.solve(*args, factor=factor, workspace=torch.empty(least, dtype=torch.uint8, device=cuda_device)))
+    for out in got:
+        for g, w in zip(out[:3], want[:3]):
+            assert torch.equal(g, w)
+    checked = engine.solve(*args, factor=factor, check_termination=5)
+    assert asked[3:] == [least] and torch.isfinite(checked[0]).all()
+    with pytest.raises(ValueError):
+        engine.solve(*args, factor=factor, workspace=torch.empty(least - 1, dtype=torch.uint8, device=cuda_device))
+    with pytest.raises(torch.OutOfMemoryError):
+        engine.solve(*args)

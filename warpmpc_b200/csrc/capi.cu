@@ -81,7 +81,7 @@ void record_stream_launch(int form, int ctas_per_sm, int grid, int smem_bytes) {
   g_last_launch[3] = smem_bytes;
 }
 
-size_t osqp_workspace_bytes(const wmpc_osqp& q, int batch, int pb, int ab, int mode, bool external);
+size_t osqp_workspace_bytes(const wmpc_osqp& q, int batch, int pb, int ab, int mode, bool external, bool least);
 size_t osqp_factor_workspace_bytes(const Osqp& o, const Pattern& pat, int pb, int ab);
 size_t osqp_adjoint_extra_bytes(const Osqp& o, int batch);
 int osqp_adjoint(const wmpc_osqp& q, const wmpc_osqp_options& opt, const wmpc_osqp_adjoint_batch& a, int mode,
@@ -1130,14 +1130,16 @@ size_t wmpc_osqp_workspace_bytes(const wmpc_osqp* osqp, int32_t batch, int32_t m
   if (!osqp || batch <= 0) return 0;
   // P/A value batches may be 1 or `batch`; size for the larger case, and
   // for the factorization-only call as well
-  const size_t solve = osqp_workspace_bytes(*osqp, batch, batch, batch, mode, external_factor != 0);
+  const size_t solve =
+      osqp_workspace_bytes(*osqp, batch, batch, batch, mode, external_factor != 0, external_factor == 2);
+  if (external_factor == 2) return solve;
   const size_t fac = osqp_factor_workspace_bytes(osqp->dev, osqp->kkt_plan->pat, batch, batch);
   return solve > fac ? solve : fac;
 }
 
 size_t wmpc_osqp_adjoint_workspace_bytes(const wmpc_osqp* osqp, int32_t batch, int32_t mode) {
   if (!osqp || batch <= 0) return 0;
-  return osqp_workspace_bytes(*osqp, batch, batch, batch, mode, false) + osqp_adjoint_extra_bytes(osqp->dev, batch);
+  return osqp_workspace_bytes(*osqp, batch, batch, batch, mode, false, false) + osqp_adjoint_extra_bytes(osqp->dev, batch);
 }
 
 int wmpc_osqp_adjoint(const wmpc_osqp* osqp, const wmpc_osqp_options* options, const wmpc_osqp_adjoint_batch* data,

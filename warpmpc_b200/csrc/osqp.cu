@@ -806,9 +806,12 @@ static bool stream_eligible(const wmpc_osqp& q, const wmpc_osqp_options* opt) {
   return q.has_stream && !env_disabled("WMPC_DISABLE_STREAM");
 }
 
-size_t osqp_workspace_bytes(const wmpc_osqp& q, int batch, int pb, int ab, int mode, bool external) {
+// least: what a solve with a given factorization cannot do without (the per-lane
+// kernel's workspace, the only one where termination is checked).
+size_t osqp_workspace_bytes(const wmpc_osqp& q, int batch, int pb, int ab, int mode, bool external, bool least) {
   size_t total = 0, total2 = 0;
   carve(q.dev, q.kkt_plan->pat, batch, pb, ab, mode, external, nullptr, &total);
+  if (least) return total;
   // a workspace sized here must serve both the streaming and the fallback kernels
   carve(q.dev, q.kkt_plan->pat, batch, pb, ab, mode, external, nullptr, &total2, &q, stream_eligible(q, nullptr));
   return total > total2 ? total : total2;

@@ -145,6 +145,11 @@ class OSQPEngine:
             return int(lib.wmpc_osqp_adjoint_workspace_bytes(self.dev.handle, batch, mode_id))
         return int(lib.wmpc_osqp_workspace_bytes(self.dev.handle, batch, mode_id, 0))
 
+    def factor_workspace_bytes(self, batch: int) -> int:
+        """Device workspace bytes that a solve of ``batch`` instances with a given
+        factorization cannot do without (it is faster with ``workspace_bytes``)."""
+        return int(native.lib().wmpc_osqp_workspace_bytes(self.dev.handle, batch, _MODES[self.mode], 2))
+
     def stream_info(self) -> dict:
         """The streaming schedule this problem carries: ``streaming`` (persistent
         solves run the streaming kernel), ``frontier_slots`` (work-vector slots
@@ -261,8 +266,14 @@ class OSQPEngine:
         or ``adjoint_workspace_bytes`` with ``keep_factor``) instead of a new
         allocation per call: a caller that chains solves (an SQP loop, a CUDA
         graph) keeps one; a kept factorization lives in it until the next
-        solve that is given the same workspace.
+        solve that is given the same workspace.  A fixed-iteration solve with
+        a given ``factor`` copies it once per instance into its workspace;
+        where that much cannot be allocated, or the given workspace holds
+        only ``factor_workspace_bytes``, and with ``check_termination``, the
+        factor is read in place (slower).
         """
+        import torch
+
         pl = self.plan
         dev = self.device
         data, opts, keep, outs, batch = self._batch_args(p_values, a_values, q, l, u, warm, max_iter,
@@ -285,19 +296,26 @@ class OSQPEngine:
         if keep_factor:
             if factor is not None:
                 raise ValueError("keep_factor needs the solve to factor (no external factor)")
-            need = lib.wmpc_osqp_adjoint_workspace_bytes(self.dev.handle, batch, mode_id)
+            need = want = lib.wmpc_osqp_adjoint_workspace_bytes(self.dev.handle, batch, mode_id)
         else:
-            need = lib.wmpc_osqp_workspace_bytes(self.dev.handle, batch, mode_id, ext)
+            need = want = lib.wmpc_osqp_workspace_bytes(self.dev.handle, batch, mode_id, ext)
+            if ext:
+                need = lib.wmpc_osqp_workspace_bytes(self.dev.handle, batch, mode_id, 2)
+                if opts.check_termination > 0:
+                    want = need
         if workspace is not None:
             if workspace.device != dev or workspace.numel() * workspace.element_size() < need:
                 raise ValueError(f"workspace must be a device tensor of at least {need} bytes on {dev}")
             ws, wsb = workspace, int(workspace.numel() * workspace.element_size())
         else:
-            ws, wsb = _workspace(need, dev)
+            try:
+                ws, wsb = _workspace(want, dev)
+            except torch.OutOfMemoryError:
+                if want <= need:
+                    raise
+                ws, wsb = _workspace(need, dev)
         if pl.settings.adaptive_rho:
             # each instance's final rho and number of rho changes (refactorizations)
-            import torch
-
             rho_out = torch.empty(batch, dtype=torch.float32, device=dev)
             upd_out = torch.empty(batch, dtype=torch.int32, device=dev)
             data.rho, data.rho_updates = rho_out.data_ptr(), upd_out.data_ptr()
