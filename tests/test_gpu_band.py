@@ -135,6 +135,26 @@ def test_band_form_choice(cuda_device):
         assert (native.stream_last_launch()["form"] == "band") == band, cls.name
 
 
+@pytest.mark.parametrize("kind,nx,nu,horizon,limit", [
+    ("small", 4, 2, 2, 0), ("small", 4, 1, 6, 0), ("small", 2, 1, 15, 0), ("small", 5, 1, 6, 0),  # short chains
+    ("quadrotor", 12, 4, 1, 148), ("small", 4, 1, 10, 148), ("small", 5, 1, 20, 148), ("small", 2, 1, 50, 148),
+    ("quadrotor", 12, 4, 10, 148), ("small", 4, 1, 20, None), ("quadrotor", 12, 4, 15, None)])
+def test_band_form_choice_by_chain(cuda_device, kind, nx, nu, horizon, limit):
+    """Up to how many tiles a pattern runs the band form by default: none for a short
+    chain, one per SM, or any number."""
+    import torch
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    cls = problems.MPCClass("x", nx, nu, horizon, 5.0, 5.0, 1.0, kind)
+    b = problems.make_batch(cls, 2, seed=1)
+    comp = compile_osqp(problems.make_plan(b), np.float32, qdldl_backend="cuda", transpose_work=True)
+    args = _dev(b.p_values, b.a_values, b.q, b.l, b.u)
+    for tiles in (1, sms, sms + 1):
+        comp.engine.solve(*[t.repeat(tiles * 16, 1) for t in args], max_iter=2)
+        band = native.stream_last_launch()["form"] == "band"
+        assert band == (limit is None or (limit > 0 and tiles <= sms)), tiles
+
+
 def test_band_form_wait_timeout(cuda_device, monkeypatch):
     """Waits limited to one microsecond give up: every instance is marked, the
     launch returns, and the next solve is right."""

@@ -378,22 +378,44 @@ bool band_wanted() {
   return !f || atoi(f) == 2;
 }
 
-// Tiles (of 32 instances) up to which a solve runs the band form.  Its fixed
-// cost is the pre-chain, whose columns and rows one warp does before the others
-// may go on (some 2.5 us per column and iteration, against 0.2 per chain row):
-// it loses where the chain is not much longer.  Where the chain is 10 to 20
-// times as long it wins only up to one tile per SM: with more, the streaming
-// form shares an SM between two tiles.  ADMM of 25 iterations, us, band
-// against streaming form, at 2000 / 9000 / 60,000 instances:
-//   20-step small class (T 79, 12)       1008 / 1483 /  9898 against  932 / 1137 /  8154
-//   10-step quadrotor class (T 121, 7)   1269 / 2557 / 16459 against 1789 / 2406 / 16627
-//   40-step small class (T 159, 12)      1500 / 3003 / 19409 against 1819 / 2599 / 17822
-//   20-step cartpole class (T 83, 4)      570 /  988 /  6654 against  892 / 1043 /  8132
-//   20-step quadrotor class (T 241, 7)   2085 / 4344 / 27593 against 3489 / 5069 / 36004
-int band_tile_limit(const BandPlan& bp, int num_sms) {
+// Tiles (of 32 instances) up to which a solve runs the band form.
+//
+// With at most one tile per SM: where a linear model of both forms' whole calls says
+// so.  Fitted to 43 patterns (MPC classes of 2 to 12 states and 1 to 80 steps, QPs
+// with one sum constraint), us for 25 iterations of 1000 instances, within 3 %
+// (streaming form) and 5 % (band form) on average; it picks the slower form for one
+// of them (by 3 %):
+//   streaming form            93 + 1.75 n + 0.45 nnz(L)
+//   band form, 8-row window  125 + 1.5 n + 1.12 T + 38 n_pre
+//              16-row window 135 +         9.4 T  + 28 n_pre
+// A pre-chain column costs most of all (one warp does them before the others may go
+// on): below ten chain rows for each the band form is not asked for.
+//
+// With more tiles the streaming form shares an SM between two of them, the band form
+// with a 16-row window does not.  There it needs a long chain, and enough entries per
+// chain row for the streaming form to be slow.  Measured, band against streaming
+// form, us at 1000 / 9000 / 30,000 instances:
+//   8 rows   4 states, 1 input, 20 steps (T  83,  4)  786 / 1341 /  4821 against 1092 / 1364 /  5383
+//            4 states, 1 input, 50 steps (T 203,  4) 1505 / 2905 / 10044 against 2579 / 3844 / 14430
+//            4 states, 2 inputs, 50 steps (T 199, 12) 2227 / 4362 / 15079 against 2713 / 4207 / 15839
+//            2 states, 1 input, 50 steps (T 196,  2) 1027 / 1746 /  6269 against 1156 / 1592 /  5804
+//            2 states, 1 input, 80 steps (T 316,  2) 1541 / 3005 / 10388 against 1788 / 2969 / 10997
+//   16 rows  4 states, 1 input, 6 steps  (T  35,  0)  471 /  860 /  2843 against  385 /  457 /  1559
+//            5 states, 1 input, 20 steps (T 104,  5) 1080 / 2084 /  7094 against 1408 / 1780 /  6956
+//            quadrotor, 10 steps         (T 121,  7) 1573 / 3113 / 10578 against 2092 / 2956 / 10822
+//            quadrotor, 15 steps         (T 181,  7) 2024 / 4144 / 13955 against 3063 / 4459 / 17173
+//            quadrotor, 30 steps         (T 361,  7) 3519 / 7072 / 24251 against 6883 / 9724 / 37242
+int band_tile_limit(const BandPlan& bp, int nnz_l, int num_sms) {
   if (getenv("WMPC_STREAM_BAND")) return INT_MAX;  // asked for
-  if (bp.T >= 20 * bp.n_pre) return INT_MAX;
-  return bp.T >= 10 * bp.n_pre ? num_sms : 0;
+  const bool wide = bp.units > 2;
+  if (bp.T < 10 * bp.n_pre) return 0;
+  const bool many = wide ? bp.T >= 150 && nnz_l >= 18LL * bp.T
+                         : bp.T >= 300 || (bp.T >= 80 && nnz_l >= 10LL * bp.T);
+  if (bp.T >= 20 * bp.n_pre && many) return INT_MAX;
+  const double stream_us = 93.0 + 1.75 * bp.n + 0.45 * nnz_l;
+  const double band_us = wide ? 135.0 + 9.4 * bp.T + 28.0 * bp.n_pre
+                              : 125.0 + 1.5 * bp.n + 1.12 * bp.T + 38.0 * bp.n_pre;
+  return band_us < stream_us ? num_sms : 0;
 }
 
 }  // namespace
@@ -1098,7 +1120,7 @@ int wmpc_osqp_create(const wmpc_osqp_desc* desc, const wmpc_plan* kkt_plan, wmpc
     q->has_band = q->has_stream && band_wanted() &&
                   build_band_plan(hp, desc, unscale, &q->bp, &q->band_factor, &q->band_block, lists, q->tile_factor[2],
                                   &why);
-    if (q->has_band) q->band_tiles = band_tile_limit(q->bp, q->num_sms);
+    if (q->has_band) q->band_tiles = band_tile_limit(q->bp, hp.nnz_l, q->num_sms);
   }
   *out = q;
   return WMPC_OK;
