@@ -311,3 +311,31 @@ def test_given_factorization_in_less_memory(cuda_device, monkeypatch):
         engine.solve(*args, factor=factor, workspace=torch.empty(least - 1, dtype=torch.uint8, device=cuda_device))
     with pytest.raises(torch.OutOfMemoryError):
         engine.solve(*args)
+
+
+@pytest.mark.parametrize("check", [0, 5])
+def test_band_form_overflowed_instances(cuda_device, monkeypatch, check):
+    """Instances whose iterates overflow are reported as in the streaming form, and their
+    tiles' other instances are untouched.  (Which of an overflowed instance's values are
+    infinite and which are NaN may differ: padding multiplies zeros with its rows.)"""
+    batch, broken = 75, [3, 40, 41, 74]
+    b = problems.make_batch(problems.CARTPOLE, batch, seed=4)
+    plan = problems.make_plan(b, OSQPSettings(**{**problems.DEFAULT_SETTINGS, "max_iter": 30}))
+    p, a, q = b.p_values.copy(), b.a_values.copy(), b.q.copy()
+    q[3, 5] = np.inf
+    q[40, :] = 3e38
+    a[41, 7] = 1e30
+    q[74, 0] = np.nan
+    band, plain = _compile(monkeypatch, plan, 1), _compile(monkeypatch, plan, 0)
+    outs, status = [], []
+    for comp in (band, plain):
+        outs.append([o.cpu().numpy() for o in comp.engine.solve(*_dev(p, a, q, b.l, b.u), check_termination=check)])
+        status.append(comp.engine.last_status.cpu().numpy())
+    np.testing.assert_array_equal(*status)
+    keep = np.setdiff1d(np.arange(batch), broken)
+    for g, w in zip(*outs):
+        np.testing.assert_array_equal(g[keep], w[keep])
+        # finite in both: the same value
+        both = np.isfinite(g) & np.isfinite(w)
+        np.testing.assert_array_equal(g[both], w[both])
+    assert np.all(status[0][[3, 40, 74]] & native.STATUS_NONFINITE)
