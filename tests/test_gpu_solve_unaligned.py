@@ -11,6 +11,22 @@ from warpmpc_b200.jax_qdldl import compile_qdldl_variant
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("nx,horizon", [(4, 2), (4, 8), (4, 20)])
+@pytest.mark.parametrize("batch", [9501, 30001, 60001])
+def test_unaligned_solve_of_short_patterns(cuda_device, monkeypatch, nx, horizon, batch):
+    """Several tiles per SM: few stages and many CTAs, or the one-lane kernel."""
+    import torch
+
+    b = problems.make_batch(problems.MPCClass("x", nx, 1, horizon, 5.0, 10.0, 2.0, "small"), 2, seed=8)
+    qp = problems.make_plan(b).qdldl_plan
+    comp = compile_qdldl_variant(qp, np.float32, backend="cuda", transpose_work=True)
+    gen = torch.Generator(device="cuda").manual_seed(batch)
+    lx, dinv, rhs = (torch.randn(k, batch, generator=gen, device="cuda") for k in (qp.nnz_l, qp.n, qp.n))
+    got = comp.solve(0.02 * lx, dinv, rhs).clone()
+    monkeypatch.setenv("WMPC_SOLVE_STREAM_OFF", "1")
+    assert torch.equal(got, comp.solve(0.02 * lx, dinv, rhs))
+
+
 @pytest.mark.parametrize("batch,shift", [(1, 0), (31, 0), (33, 1), (64, 1), (4803, 0)])
 def test_unaligned_solve_matches_one_lane(cuda_device, monkeypatch, batch, shift):
     import torch

@@ -8,8 +8,8 @@
 // bulk copy of the item's index table; an mbarrier per stage signals arrival.
 // Where the batch or an array does not meet the tensor copies' 16-byte rule, the
 // producer copies the same rows with 4-byte asynchronous copies instead, one row
-// of 32 lanes each (4097 instances of the
-// 30-step quadrotor class 0.82 ms, where the one-lane kernel took 3.70 ms).
+// of 32 lanes each (4097 instances of the 30-step quadrotor class 0.82 ms, where
+// the one-lane kernel took 3.70 ms).
 // The other warp (the sweeper) works on the stage from shared memory:
 //   rhs items      rows of rhs in natural order, scattered into the work
 //                  vector X through pinv (X = P rhs);
@@ -403,11 +403,38 @@ bool build_solve_tables(int n, const std::vector<int>& lp, const std::vector<int
   return true;
 }
 
+// Stages of a launch fed by 4-byte copies: as many as leave room for the CTAs that
+// the tiles ask for, two at least.  The sweeper's latency bounds a CTA, not its
+// feed: with one tile per SM 2 stages take as long as 8 (30-step quadrotor class 2 %
+// longer), and short patterns get up to seven CTAs on an SM.  0: the one-lane kernel
+// is the faster one, for patterns so short that it has every instance in flight
+// where this one takes a third round of tiles.  us, eight stages / this rule /
+// one-lane kernel, repeated solves and (in brackets) with a cold L2:
+//   126 rows, 30,001 instances   281 (285) / 103 (111) / 121 (195)
+//   172 rows, 15,001             222 (227) /  73  (78) / 173 (274)
+//   222 rows, 60,001             941 (944) / 390 (397) / 805 (815)
+//    60 rows, 30,001              84  (88) /  52  (59) /  60  (90)
+//    60 rows, 60,001             147 (156) /  83  (94) /  62  (94): the one-lane kernel
+int unaligned_stages(int n, int batch, int most, int num_sms, int sm_total, int reserved) {
+  const int tiles = (batch + 31) / 32;
+  auto resident = [&](int stages) { return std::min(32, sm_total / ((int)solve_smem_bytes(n, stages) + reserved)); };
+  const int want = std::min((tiles + num_sms - 1) / num_sms, resident(2));
+  int stages = most;
+  while (stages > 2 && resident(stages) < want) --stages;
+  const int threads = std::min(128, smem_lanes_for_rows(n));
+  if (threads >= 32 && tiles > 2 * num_sms * std::max(resident(stages), 1)) {
+    const int blocks = std::min(2048 / threads, sm_total / (4 * n * threads + reserved));
+    if (batch <= (long long)blocks * num_sms * threads) return 0;
+  }
+  return stages;
+}
+
 // The streamed solve when it applies: one factor per instance (fstride 1, or one
-// instance), the plan's chunk tables built, and the work vector plus two stages in shared
-// memory; fed by tensor copies where the batch is a multiple of 4 (16-byte row
-// pitch) and the arrays are 16-byte aligned, else by 4-byte copies.  *applied is false when it did not apply (the caller then runs
-// the one-lane kernel); the return value is a WMPC status.
+// instance), the plan's chunk tables built, and the work vector plus two stages in
+// shared memory; fed by tensor copies where the batch is a multiple of 4 (16-byte row
+// pitch) and the arrays are 16-byte aligned, else by 4-byte copies.  *applied is
+// false when it did not apply (the caller then runs the one-lane kernel); the return
+// value is a WMPC status.
 int launch_solve_stream(const wmpc_plan& plan, const float* lx, const float* dinv, int fstride, const float* rhs,
                         float* x, int batch, cudaStream_t s, bool* applied) {
   const Pattern& pat = plan.pat;
@@ -426,6 +453,16 @@ int launch_solve_stream(const wmpc_plan& plan, const float* lx, const float* din
   int stages = kMaxStages;
   while (stages >= 2 && solve_smem_bytes(pat.n, stages) > (size_t)sm_bytes) --stages;
   if (stages < 2) return WMPC_OK;
+  if (!tma) {
+    int sm_total = 0, reserved = 0;
+    if (cudaDeviceGetAttribute(&sm_total, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return WMPC_OK;
+    }
+    stages = unaligned_stages(pat.n, batch, stages, num_sms, sm_total, reserved);
+    if (stages == 0) return WMPC_OK;
+  }
   SolveArgs a{};
   if (tma && (!encode_rows(&a.tm_l, lx, pat.nnz_l, batch) || !encode_rows(&a.tm_d, dinv, pat.n, batch) ||
       !encode_rows(&a.tm_r, rhs, pat.n, batch)))
