@@ -153,6 +153,9 @@ def test_band_form_choice_by_chain(cuda_device, kind, nx, nu, horizon, limit):
         comp.engine.solve(*[t.repeat(tiles * 16, 1) for t in args], max_iter=2)
         band = native.stream_last_launch()["form"] == "band"
         assert band == (limit is None or (limit > 0 and tiles <= sms)), tiles
+    comp.engine.solve(*[t.repeat((sms + 1) * 16, 1) for t in args], max_iter=2, check_termination=1)
+    band = native.stream_last_launch()["form"] == "band"
+    assert band == (limit is None and (kind, horizon) != ("small", 20))
 
 
 def test_band_form_wait_timeout(cuda_device, monkeypatch):

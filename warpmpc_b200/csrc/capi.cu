@@ -405,12 +405,15 @@ bool band_wanted() {
 //            quadrotor, 10 steps         (T 121,  7) 1573 / 3113 / 10578 against 2092 / 2956 / 10822
 //            quadrotor, 15 steps         (T 181,  7) 2024 / 4144 / 13955 against 3063 / 4459 / 17173
 //            quadrotor, 30 steps         (T 361,  7) 3519 / 7072 / 24251 against 6883 / 9724 / 37242
-int band_tile_limit(const BandPlan& bp, int nnz_l, int num_sms) {
+// With termination checks two CTAs share an SM less well in the band form: the 20-step
+// class of 4 states and 1 input takes 831 / 1700 / 6072 against 1255 / 1421 / 5326, the
+// 50-step class 1583 / 3519 / 11950 against 2988 / 4256 / 16367.
+int band_tile_limit(const BandPlan& bp, int nnz_l, bool check, int num_sms) {
   if (getenv("WMPC_STREAM_BAND")) return INT_MAX;  // asked for
   const bool wide = bp.units > 2;
   if (bp.T < 10 * bp.n_pre) return 0;
   const bool many = wide ? bp.T >= 150 && nnz_l >= 18LL * bp.T
-                         : bp.T >= 300 || (bp.T >= 80 && nnz_l >= 10LL * bp.T);
+                         : bp.T >= 300 || (bp.T >= (check ? 150 : 80) && nnz_l >= 10LL * bp.T);
   if (bp.T >= 20 * bp.n_pre && many) return INT_MAX;
   const double stream_us = 93.0 + 1.75 * bp.n + 0.45 * nnz_l;
   const double band_us = wide ? 135.0 + 9.4 * bp.T + 28.0 * bp.n_pre
@@ -1120,7 +1123,8 @@ int wmpc_osqp_create(const wmpc_osqp_desc* desc, const wmpc_plan* kkt_plan, wmpc
     q->has_band = q->has_stream && band_wanted() &&
                   build_band_plan(hp, desc, unscale, &q->bp, &q->band_factor, &q->band_block, lists, q->tile_factor[2],
                                   &why);
-    if (q->has_band) q->band_tiles = band_tile_limit(q->bp, hp.nnz_l, q->num_sms);
+    for (int check = 0; check < 2 && q->has_band; ++check)
+      q->band_tiles[check] = band_tile_limit(q->bp, hp.nnz_l, check != 0, q->num_sms);
   }
   *out = q;
   return WMPC_OK;

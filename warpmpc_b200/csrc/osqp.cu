@@ -925,7 +925,7 @@ int stream_solve_begin(const wmpc_osqp& q, const wmpc_osqp_options& opt, const w
   return WMPC_OK;
 }
 
-bool band_for(const wmpc_osqp& q, int tiles) { return q.has_band && tiles <= q.band_tiles; }
+bool band_for(const wmpc_osqp& q, bool check, int tiles) { return q.has_band && tiles <= q.band_tiles[check ? 1 : 0]; }
 
 // The band form's first half: inputs staged, factor, state records; fills `job`.
 int band_prepare(const wmpc_osqp& q, const wmpc_osqp_options& opt, const wmpc_osqp_batch& d, const Layout& L,
@@ -994,7 +994,7 @@ int stream_solve_adaptive(const wmpc_osqp& q, const wmpc_osqp_options& opt, cons
   WMPC_LAUNCH_CHECK();
   State st{L.x, L.z, L.y, L.qs, L.ls, L.us, B};
   BandJobDesc band;
-  const bool use_band = band_for(q, (B + 31) / 32);
+  const bool use_band = band_for(q, false, (B + 31) / 32);
   auto begin = [&](bool warm, const int* only) -> int {
     if (use_band) {
       const int r = band_prepare(q, opt, d, L, warm, false, &band, s, L.rinv_row, only);
@@ -1112,9 +1112,9 @@ int osqp_solve(const wmpc_osqp& q, const wmpc_osqp_options& opt, const wmpc_osqp
   if (L.streaming && adaptive) {
     StreamJobDesc job;
     if ((rc = stream_solve_adaptive(q, opt, d, L, &job, s))) return rc;
-    return stream_solve_end(q, opt, d, L, band_for(q, (B + 31) / 32) ? nullptr : &job, L.error_word, s);
+    return stream_solve_end(q, opt, d, L, band_for(q, false, (B + 31) / 32) ? nullptr : &job, L.error_word, s);
   }
-  if (L.streaming && band_for(q, (B + 31) / 32)) {
+  if (L.streaming && band_for(q, opt.check_termination > 0, (B + 31) / 32)) {
     BandJobDesc job;
     if ((rc = band_solve_begin(q, opt, d, L, &job, s, given))) return rc;
     if ((rc = band_run(&job, 1, L.error_word, q.num_sms, s))) return rc;
@@ -1272,7 +1272,7 @@ int osqp_solve_multi(const wmpc_osqp* const* qs, const wmpc_osqp_options* opts, 
     if (ds[i].batch > 0) {
       const double work = (double)((ds[i].batch + 31) / 32) * qs[i]->kkt_plan->pat.nnz_l;
       all_work += work;
-      if (band_for(*qs[i], tiles)) band_work_part += work;
+      if (band_for(*qs[i], opts[i].check_termination > 0, tiles)) band_work_part += work;
       band = band && qs[i]->has_band;
       plans.push_back(&qs[i]->bp);
       frontier = frontier && frontier_for(*qs[i], opts[i].check_termination > 0, tiles);

@@ -80,8 +80,9 @@ struct wmpc_osqp {
   wmpc::StreamPlan spf{};
   void* stream_block_f = nullptr;
   // the band form (band.cuh): run by persistent solves of at most band_tiles tiles
+  // ([1]: with termination checks)
   bool has_band = false;
-  int band_tiles = 0;
+  int band_tiles[2] = {0, 0};
   wmpc::BandPlan bp{};
   wmpc::StreamPlan band_factor{};  // the factorization's tables, writing the band form's stream
   void* band_block = nullptr;
