@@ -231,7 +231,8 @@ __device__ __forceinline__ void chain_forward(float (&A)[4 * MU + kTurn], const 
   chain_load<MU>(lst, w.x, L[0]);
 #pragma unroll 1
   for (int t = 0; t < cols; t += kTurn) {
-    const int4 wn = *reinterpret_cast<const int4*>(words + (t + kTurn < cols ? t + kTurn : 0));  // (past the end: not used)
+    // (past the end: not used)
+    const int4 wn = *reinterpret_cast<const int4*>(words + (t + kTurn < cols ? t + kTurn : 0));
 #pragma unroll
     for (int p = 0; p < kTurn; ++p) {
       chain_load<MU>(lst, p < kTurn - 1 ? comp4(w, p + 1) : wn.x, L[(p + 1) & 1]);
@@ -412,9 +413,10 @@ __global__ void __launch_bounds__(kWide ? 512 : 640, 1) band_admm_kernel(const _
   unsigned* b_done = chain_done + 1;
   unsigned* pre_b = chain_done + 2;
   unsigned* pre_f = chain_done + 3;
-  volatile int* skip_to = reinterpret_cast<volatile int*>(chain_done + 4);  // tiles (of this CTA) before this one are over
-  volatile int* tag = reinterpret_cast<volatile int*>(chain_done + 5);      // [stages] tile ordinal of a stage's copy
-  unsigned* f_done = chain_done + 5 + a.stages;                             // [K]
+  // tiles (of this CTA) before this one are over; [stages] tile ordinal of a stage's copy; [K]
+  volatile int* skip_to = reinterpret_cast<volatile int*>(chain_done + 4);
+  volatile int* tag = reinterpret_cast<volatile int*>(chain_done + 5);
+  unsigned* f_done = chain_done + 5 + a.stages;
   const int total = a.tile_end[a.n_jobs - 1];
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2 * a.stages; ++s) mbar_init(cfull + s, 1);
@@ -1057,7 +1059,8 @@ bool band_fits(const BandPlan* const* plans, int n) {
 
 // One launch over every class's tiles, the costliest class first.
 int band_run(const BandJobDesc* jobs, int n_jobs, int* error, int num_sms, cudaStream_t s) {
-  if (n_jobs < 1 || n_jobs > kMaxBandJobs) return fail(WMPC_ERR_INVALID_ARGUMENT, "1 to %d classes per launch", kMaxBandJobs);
+  if (n_jobs < 1 || n_jobs > kMaxBandJobs)
+    return fail(WMPC_ERR_INVALID_ARGUMENT, "1 to %d classes per launch", kMaxBandJobs);
   bool track = false, rho = false;
   int order[kMaxBandJobs], limit = jobs[0].ctas_limit, total = 0;
   double cost[kMaxBandJobs];

@@ -53,7 +53,8 @@ struct BandPlan {
   int item_bytes;               // the largest item
   int n_rows;                   // 128-byte rows of records
   const int* col_word;   // [T4] 1: the last unit is there too | first unit in the chunk << 1
-  const int4* chunk;     // [n_chunks] {float offset, bytes before D^-1, columns | far entries << 8, chain rows its forward pass needs}
+  const int4* chunk;     // [n_chunks] {float offset, bytes before D^-1, columns | far entries << 8, chain rows
+                         // that its forward pass needs}
   const int* far_ptr;    // [n_chunks] first far entry
   const int4* far;       // {column in its chunk, work-vector byte offset of its row, byte offset in the chunk, 0}
   const int* item;       // [2 n_pre + nb + T] stream offset in 128-byte rows | rows << 22
@@ -63,16 +64,15 @@ struct BandPlan {
   const int* param_off;  // [n] by original KKT index: stream offset of its parameter record
 };
 // Items: pre-chain columns (last first), subtrees, pre-chain rows, chain rows.  A
-// record
-// (32-bit words).  Pre-chain column or subtree: {units | children << 4 | kinds
-// << 8, 12, 16 (root, children) | record rows << 27, forward-result byte offset, chunks
-// needed | kBandUsesPre, solution byte offset of a pre-chain column, or stream
-// offset of the root's D^-1}, {rho, 1/rho, unscale, residual offset} of the root
-// and of two children, then the work-vector byte offset of every entry.  Row:
-// {units | kind << 8 | kBandUsesPre | record rows << 27, work-vector byte offset,
-// forward-result byte offset of a pre-chain row or -1, stream offset of its
-// parameters}, {rho, 1/rho, unscale, residual offset}, then the forward-result
-// byte offset of every entry.  A kind: bit 0 constraint, bits 1-2 its rho class + 1.
+// record (32-bit words) of a pre-chain column or subtree: {units | children << 4 |
+// kinds << 8, 12, 16 (root, children) | record rows << 27, forward-result byte
+// offset, chunks needed | kBandUsesPre, solution byte offset of a pre-chain column,
+// or stream offset of the root's D^-1}, {rho, 1/rho, unscale, residual offset} of
+// the root and of two children, then the work-vector byte offset of every entry.  Of
+// a row: {units | kind << 8 | kBandUsesPre | record rows << 27, work-vector byte
+// offset, forward-result byte offset of a pre-chain row or -1, stream offset of its
+// parameters}, {rho, 1/rho, unscale, residual offset}, then the forward-result byte
+// offset of every entry.  A kind: bit 0 constraint, bits 1-2 its rho class + 1.
 constexpr int kBandRecB = 16, kBandRecF = 8;  // words before the entries' offsets
 
 struct HostBand {

@@ -119,16 +119,16 @@ struct wmpc_plan {
   const int* solve_tables = nullptr;
   const int* solve_desc = nullptr;  // two int4 per chunk
   int solve_chunks = 0;
-  // compact-accumulator tables of the staged per-call factorization (null:
-  // the one-lane kernel factors): slot of each initial entry in its row's
-  // reach, per program entry its range of updates, per update its target
-  // slot and the L entry it re-reads
   // the tile factorization (tile_factor.cuh): its lists for the per-call factor, its schedule
   const int4* tile_prog = nullptr;
   const int* tile_off = nullptr;
   int tile_slots = 0;
   std::shared_ptr<wmpc::HostTileSchedule> h_tile;
   std::vector<int> h_init_slot;
+  // compact-accumulator tables of the staged per-call factorization (null:
+  // the one-lane kernel factors): slot of each initial entry in its row's
+  // reach, per program entry its range of updates, per update its target
+  // slot and the L entry it re-reads
   const int* fac_init_slot = nullptr;
   const int* fac_upd_ptr = nullptr;
   const int* fac_upd_slot = nullptr;

@@ -790,7 +790,8 @@ int stream_begin(const Pattern& pat, const StreamPlan& sp, const Osqp& o, const 
                  const float* aT, long long lda, int sba, const float* x, const float* z, const float* y,
                  const float* qs, const float* ls, const float* us, bool warm, bool track, float* work,
                  int* status, int batch, int num_sms, bool reuse_factor, StreamJobDesc* job, cudaStream_t s,
-                 const TileFactor* tf, const float* rinv_rows = nullptr, const int* only = nullptr, const ExternalFactor* given = nullptr);
+                 const TileFactor* tf, const float* rinv_rows = nullptr, const int* only = nullptr,
+                 const ExternalFactor* given = nullptr);
 int stream_import(const Pattern& pat, const StreamPlan& sp, const ExternalFactor& f, float* bstream, float* fstream,
                   int* status, int batch, cudaStream_t s);
 int stream_factor(const Pattern& pat, const StreamPlan& sp, const Osqp& o, const float* pT, long long ldp, int sbp,
@@ -1005,8 +1006,8 @@ int stream_solve_adaptive(const wmpc_osqp& q, const wmpc_osqp_options& opt, cons
       return r;
     }
     int r = stream_begin(q.kkt_plan->pat, sp, o, L.pT, pb, sbp, L.aT, ab, sba, L.x, L.z, L.y, L.qs, L.ls, L.us, warm,
-                         false, L.stream_ws, L.stream_status, B, q.num_sms, false, job, s, q.tile_factor[frontier ? 1 : 0],
-                         L.rinv_row, only);
+                         false, L.stream_ws, L.stream_status, B, q.num_sms, false, job, s,
+                         q.tile_factor[frontier ? 1 : 0], L.rinv_row, only);
     job->check_every = 0;
     job->ctas_limit = q.ctas_limit;
     job->chg_eps = opt.eps_abs;
@@ -1028,9 +1029,9 @@ int stream_solve_adaptive(const wmpc_osqp& q, const wmpc_osqp_options& opt, cons
       if ((rc = use_band ? band_state_out(q.bp, band_work(q.bp, B, L.stream_ws), L.x, L.z, L.y, B, s)
                          : stream_end(sp, o, *job, L.x, L.z, L.y, s)))
         return rc;
-      rho_update_kernel<<<ceil_div(B, 32), dim3(32, kRhoParts), 0, s>>>(o, L.pT, pb, sbp, L.aT, ab, sba, st, L.rho_row, L.rinv_row,
-                                                         L.rho_b, L.rho_changed, L.rho_count,
-                                                         opt.adaptive_rho_tolerance, B);
+      rho_update_kernel<<<ceil_div(B, 32), dim3(32, kRhoParts), 0, s>>>(
+          o, L.pT, pb, sbp, L.aT, ab, sba, st, L.rho_row, L.rinv_row, L.rho_b, L.rho_changed, L.rho_count,
+          opt.adaptive_rho_tolerance, B);
       WMPC_LAUNCH_CHECK();
       if ((rc = begin(true, L.rho_changed))) return rc;
     }
@@ -1176,9 +1177,9 @@ int osqp_solve(const wmpc_osqp& q, const wmpc_osqp_options& opt, const wmpc_osqp
       if (adaptive && (it + 1) % opt.adaptive_rho_interval == 0 && it + 1 < opt.max_iter) {
         // new rho estimates; the instances whose rho changed refactor, and
         // every instance's next right-hand side is formed with its rho
-        rho_update_kernel<<<ceil_div(B, 32), dim3(32, kRhoParts), 0, s>>>(o, L.pT, ldp, sbp, L.aT, lda, sba, st, L.rho_row,
-                                                           L.rinv_row, L.rho_b, L.rho_changed, L.rho_count,
-                                                           opt.adaptive_rho_tolerance, B);
+        rho_update_kernel<<<ceil_div(B, 32), dim3(32, kRhoParts), 0, s>>>(
+            o, L.pT, ldp, sbp, L.aT, lda, sba, st, L.rho_row, L.rinv_row, L.rho_b, L.rho_changed, L.rho_count,
+            opt.adaptive_rho_tolerance, B);
         WMPC_LAUNCH_CHECK();
         assemble_kkt_rho_kernel<<<kgrid, 128, 0, s>>>(o, L.pT, ldp, sbp, L.aT, lda, sba, L.rinv_row, L.rho_changed,
                                                       L.kkt, B);

@@ -116,103 +116,103 @@ bool schedule_tile_factor(const HostPattern& hp, const std::vector<int>& init_sl
   // ---- schedule ----
   const int W = kTfWarps;
   auto schedule = [&](int look, std::vector<int> npred, HostTileSchedule* result) -> bool {
-  HostTileSchedule& H = *result;
-  std::vector<int> tick(N, -1), warp(N, -1), load_tick(n, -1), dep_tick(N, -1), dep_warp(N, -1);
-  auto& ops = H.ops;
-  ops.assign(W, {});
-  struct Ready {
-    int tail, task, warp;  // warp -1: any
-    bool operator<(const Ready& o) const { return tail != o.tail ? tail < o.tail : task > o.task; }
-  };
-  std::vector<Ready> next;                      // ready from the next tick on
-  std::vector<std::vector<Ready>> later(kTfDelay + 1);  // inits, by tick modulo
-  int done = 0, at_row = 0, at_late = 0, t = 0;
-  for (; done < N; ++t) {
-    if (t > 64 * N) {
-      *why = "the factorization's schedule does not end";
-      return false;
-    }
-    std::priority_queue<Ready> ready(std::less<Ready>(), std::move(next));
-    next.clear();
-    for (const Ready& r : later[t % (kTfDelay + 1)]) ready.push(r);
-    later[t % (kTfDelay + 1)].clear();
-    std::vector<int> load(W, 0);
-    while (!ready.empty()) {
-      const Ready r = ready.top();
-      ready.pop();
-      int w = r.warp;
-      if (w < 0) w = static_cast<int>(std::min_element(load.begin(), load.end()) - load.begin());
-      if (load[w] > 0 && load[w] + cost[r.task] > kTfTick) {
-        next.push_back({r.tail, r.task, r.task >= S ? r.warp : -1});
-        continue;
+    HostTileSchedule& H = *result;
+    std::vector<int> tick(N, -1), warp(N, -1), load_tick(n, -1), dep_tick(N, -1), dep_warp(N, -1);
+    auto& ops = H.ops;
+    ops.assign(W, {});
+    struct Ready {
+      int tail, task, warp;  // warp -1: any
+      bool operator<(const Ready& o) const { return tail != o.tail ? tail < o.tail : task > o.task; }
+    };
+    std::vector<Ready> next;                      // ready from the next tick on
+    std::vector<std::vector<Ready>> later(kTfDelay + 1);  // inits, by tick modulo
+    int done = 0, at_row = 0, at_late = 0, t = 0;
+    for (; done < N; ++t) {
+      if (t > 64 * N) {
+        *why = "the factorization's schedule does not end";
+        return false;
       }
-      load[w] += cost[r.task];
-      tick[r.task] = t;
-      warp[r.task] = w;
-      ops[w].push_back({t, r.task});
-      ++done;
-      for (int s : succ[r.task]) {
-        if (dep_tick[s] == t && dep_warp[s] != w) dep_warp[s] = -2;
-        else dep_warp[s] = w;
-        dep_tick[s] = t;
-        if (--npred[s] > 0) continue;
-        if (dep_warp[s] >= 0) ready.push({tail[s], s, w});  // the same warp may go on at once
-        else next.push_back({tail[s], s, -1});
+      std::priority_queue<Ready> ready(std::less<Ready>(), std::move(next));
+      next.clear();
+      for (const Ready& r : later[t % (kTfDelay + 1)]) ready.push(r);
+      later[t % (kTfDelay + 1)].clear();
+      std::vector<int> load(W, 0);
+      while (!ready.empty()) {
+        const Ready r = ready.top();
+        ready.pop();
+        int w = r.warp;
+        if (w < 0) w = static_cast<int>(std::min_element(load.begin(), load.end()) - load.begin());
+        if (load[w] > 0 && load[w] + cost[r.task] > kTfTick) {
+          next.push_back({r.tail, r.task, r.task >= S ? r.warp : -1});
+          continue;
+        }
+        load[w] += cost[r.task];
+        tick[r.task] = t;
+        warp[r.task] = w;
+        ops[w].push_back({t, r.task});
+        ++done;
+        for (int s : succ[r.task]) {
+          if (dep_tick[s] == t && dep_warp[s] != w) dep_warp[s] = -2;
+          else dep_warp[s] = w;
+          dep_tick[s] = t;
+          if (--npred[s] > 0) continue;
+          if (dep_warp[s] >= 0) ready.push({tail[s], s, w});  // the same warp may go on at once
+          else next.push_back({tail[s], s, -1});
+        }
+      }
+      while (at_late < N && tick[by_late[at_late]] >= 0) ++at_late;
+      const int front = at_late < N ? late(by_late[at_late]) : total;
+      for (; at_row < n && late(S + rows[at_row]) <= front + look; ++at_row) {
+        const int k = rows[at_row], ni = 1 + hp.init_ptr[k + 1] - hp.init_ptr[k];
+        const int w = static_cast<int>(std::min_element(load.begin(), load.end()) - load.begin());
+        if (load[w] > kTfTick) break;
+        load[w] += 20 + 12 * ni;
+        load_tick[k] = t;
+        ops[w].push_back({t, N + k});
+        later[(t + kTfDelay) % (kTfDelay + 1)].push_back({tail[S + k], S + k, w});
       }
     }
-    while (at_late < N && tick[by_late[at_late]] >= 0) ++at_late;
-    const int front = at_late < N ? late(by_late[at_late]) : total;
-    for (; at_row < n && late(S + rows[at_row]) <= front + look; ++at_row) {
-      const int k = rows[at_row], ni = 1 + hp.init_ptr[k + 1] - hp.init_ptr[k];
-      const int w = static_cast<int>(std::min_element(load.begin(), load.end()) - load.begin());
-      if (load[w] > kTfTick) break;
-      load[w] += 20 + 12 * ni;
-      load_tick[k] = t;
-      ops[w].push_back({t, N + k});
-      later[(t + kTfDelay) % (kTfDelay + 1)].push_back({tail[S + k], S + k, w});
+    H.ticks = t;
+    // ---- slots ----
+    struct Value {
+      int from, to, id;  // id: step e: its row's slot, S + k: d of row k
+    };
+    std::vector<Value> values;
+    std::vector<int> last_y(tick.begin(), tick.begin() + S), last_d(n);
+    for (int k = 0; k < n; ++k) last_d[k] = tick[end_of(k)];
+    for (int e = 0; e < S; ++e) {
+      last_d[hp.proc_cols[e]] = std::max(last_d[hp.proc_cols[e]], tick[e]);
+      for (const auto& u : upd[e]) last_y[u.second] = std::max(last_y[u.second], tick[e]);
     }
-  }
-  H.ticks = t;
-  // ---- slots ----
-  struct Value {
-    int from, to, id;  // id: step e: its row's slot, S + k: d of row k
-  };
-  std::vector<Value> values;
-  std::vector<int> last_y(tick.begin(), tick.begin() + S), last_d(n);
-  for (int k = 0; k < n; ++k) last_d[k] = tick[end_of(k)];
-  for (int e = 0; e < S; ++e) {
-    last_d[hp.proc_cols[e]] = std::max(last_d[hp.proc_cols[e]], tick[e]);
-    for (const auto& u : upd[e]) last_y[u.second] = std::max(last_y[u.second], tick[e]);
-  }
-  for (int k = 0; k < n; ++k) {
-    std::vector<char> has(hp.proc_ptr[k + 1] - hp.proc_ptr[k], 0);
-    for (int i = hp.init_ptr[k]; i < hp.init_ptr[k + 1]; ++i) has[init_slot[i]] = 1;
-    for (int e = hp.proc_ptr[k]; e < hp.proc_ptr[k + 1]; ++e)
-      values.push_back({has[e - hp.proc_ptr[k]] ? load_tick[k] : tick[S + k], last_y[e], e});
-    values.push_back({load_tick[k], last_d[k], S + k});
-  }
-  std::stable_sort(values.begin(), values.end(), [](const Value& a, const Value& b) { return a.from < b.from; });
-  std::vector<int> spare;
-  auto& slot = H.slot;
-  slot.assign(S + n, 0);
-  std::priority_queue<std::pair<int, int>, std::vector<std::pair<int, int>>, std::greater<std::pair<int, int>>> busy;
-  H.slots = 1;
-  for (const Value& v : values) {
-    while (!busy.empty() && busy.top().first < v.from) {
-      spare.push_back(busy.top().second);
-      busy.pop();
+    for (int k = 0; k < n; ++k) {
+      std::vector<char> has(hp.proc_ptr[k + 1] - hp.proc_ptr[k], 0);
+      for (int i = hp.init_ptr[k]; i < hp.init_ptr[k + 1]; ++i) has[init_slot[i]] = 1;
+      for (int e = hp.proc_ptr[k]; e < hp.proc_ptr[k + 1]; ++e)
+        values.push_back({has[e - hp.proc_ptr[k]] ? load_tick[k] : tick[S + k], last_y[e], e});
+      values.push_back({load_tick[k], last_d[k], S + k});
     }
-    int s;
-    if (spare.empty()) {
-      s = H.slots++;
-    } else {
-      s = spare.back();
-      spare.pop_back();
+    std::stable_sort(values.begin(), values.end(), [](const Value& a, const Value& b) { return a.from < b.from; });
+    std::vector<int> spare;
+    auto& slot = H.slot;
+    slot.assign(S + n, 0);
+    std::priority_queue<std::pair<int, int>, std::vector<std::pair<int, int>>, std::greater<std::pair<int, int>>> busy;
+    H.slots = 1;
+    for (const Value& v : values) {
+      while (!busy.empty() && busy.top().first < v.from) {
+        spare.push_back(busy.top().second);
+        busy.pop();
+      }
+      int s;
+      if (spare.empty()) {
+        s = H.slots++;
+      } else {
+        s = spare.back();
+        spare.pop_back();
+      }
+      slot[v.id] = s;
+      busy.push({v.to, s});
     }
-    slot[v.id] = s;
-    busy.push({v.to, s});
-  }
-  return true;
+    return true;
   };
   // Rows that start early keep every warp busy and take slots: as early as the
   // slots of two CTAs per SM allow, else of one.
