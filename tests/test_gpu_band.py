@@ -125,6 +125,30 @@ def test_band_form_classes(cuda_device, monkeypatch, check):
             np.testing.assert_array_equal(g.cpu().numpy(), w.cpu().numpy())
 
 
+def test_band_form_beside_a_tuned_class(cuda_device, monkeypatch):
+    """A class compiled with schedule knobs runs them alone; in a launch whose other
+    classes hold most of the work it runs the band form with them."""
+    specs, work, alone = [(problems.QUADROTOR, 500), (problems.SMALL, 700)], [], []
+    for k, (cls, batch) in enumerate(specs):
+        b = problems.make_batch(cls, batch, seed=40 + k)
+        with monkeypatch.context() as m:
+            if cls is problems.SMALL:
+                m.setenv("WMPC_STREAM_FRONTIER_COPIES", "1")
+            comp = compile_osqp(problems.make_plan(b), np.float32, qdldl_backend="cuda", transpose_work=True)
+        args = _dev(b.p_values, b.a_values, b.q, b.l, b.u)
+        alone.append([o.clone() for o in comp.engine.solve(*args)])
+        form = native.stream_last_launch()["form"]
+        assert (form == "band") == (cls is problems.QUADROTOR)
+        work.append((comp.engine, *args, None))
+    outs = solve_classes(work)
+    assert native.stream_last_launch()["form"] == "band"
+    for out, want in zip(outs, alone):
+        for g, w in zip(out[:3], want[:3]):
+            np.testing.assert_array_equal(g.cpu().numpy(), w.cpu().numpy())
+    solve_classes(work[1:])
+    assert native.stream_last_launch()["form"] != "band"
+
+
 def test_band_form_choice(cuda_device):
     """Which form a solve runs by default: long chains the band form, others
     the streaming forms where one tile per SM does not bound them."""

@@ -366,16 +366,24 @@ bool build_band_plan(const HostPattern& hp, const wmpc_osqp_desc* desc, const st
   return true;
 }
 
-// Schedule knobs in the environment ask for the unit schedules of the
-// streaming form; WMPC_STREAM_BAND=0 / 1 turns the band form off / on.
+// WMPC_STREAM_BAND=0 / 1 turns the band form off / on; a schedule form chosen with
+// WMPC_STREAM_FRONTIER turns it off.
 bool band_wanted() {
   if (const char* v = getenv("WMPC_STREAM_BAND")) return atoi(v) != 0;
+  const char* f = getenv("WMPC_STREAM_FRONTIER");
+  return !f || atoi(f) == 2;
+}
+
+// Schedule knobs in the environment ask for the unit schedules of the streaming form.
+// The problem's own solves run them; a launch of several classes may still run the
+// band form where the others hold most of its work (one class of four tuned so cost
+// such a launch of 131,072 instances the band form: 125 ms a step became 191).
+bool unit_schedule_wanted() {
   for (const char* k : {"WMPC_STREAM_UNITS", "WMPC_STREAM_COLS", "WMPC_STREAM_REL", "WMPC_STREAM_FUNITS",
                         "WMPC_STREAM_OFFLOAD", "WMPC_STREAM_LSTAGES", "WMPC_STREAM_SSTAGES",
                         "WMPC_STREAM_FRONTIER_LAG", "WMPC_STREAM_FRONTIER_COPIES"})
-    if (getenv(k)) return false;
-  const char* f = getenv("WMPC_STREAM_FRONTIER");
-  return !f || atoi(f) == 2;
+    if (getenv(k)) return true;
+  return false;
 }
 
 // Tiles (of 32 instances) up to which a solve runs the band form.
@@ -410,6 +418,7 @@ bool band_wanted() {
 // 50-step class 1583 / 3519 / 11950 against 2988 / 4256 / 16367.
 int band_tile_limit(const BandPlan& bp, int nnz_l, bool check, int num_sms) {
   if (getenv("WMPC_STREAM_BAND")) return INT_MAX;  // asked for
+  if (unit_schedule_wanted()) return 0;
   const bool wide = bp.units > 2;
   if (bp.T < 10 * bp.n_pre) return 0;
   const bool many = wide ? bp.T >= 150 && nnz_l >= 18LL * bp.T
