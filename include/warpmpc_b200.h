@@ -373,7 +373,7 @@ int wmpc_band_item_fence_host(int32_t mb, int32_t mf);
  * (warpmpc_b200/csrc/tile_factor.cuh), built on the host: no device needed.
  * out: [warps, delay, slots, ticks, words] piece_wait[delay + 1] warp_off[warps]
  * prog[words]; piece_wait: copy groups that may be under way when a list goes on at
- * a piece asked for that many ticks earlier (-1: not even this tick's copies). */
+ * a piece asked for that many ticks earlier (-1: no copy at all). */
 int wmpc_tile_factor_host(const wmpc_pattern_desc* desc, int32_t* out, int64_t out_capacity, int64_t* out_words);
 
 /* Profiling (no counterpart in the reference, which times with wall

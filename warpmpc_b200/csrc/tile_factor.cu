@@ -180,9 +180,7 @@ tile_factor_kernel(TileFactor tf, TileFactorOut out, const float* __restrict__ s
       } else {
         if (h.y) break;
         // the next piece was asked for when the last but two was entered
-        const int under_way = tf_piece_wait(tick - entered[2]);
-        if (under_way == kTfDelay - 1) cp_async_wait_group<kTfDelay - 1>();
-        else if (under_way == 0) cp_async_wait_group<0>();
+        if (tf_piece_wait(tick - entered[2]) == kTfDelay - 1) cp_async_wait_group<kTfDelay - 1>();
         else cp_async_wait_all();
         __syncwarp();
         fetch(piece + 4);

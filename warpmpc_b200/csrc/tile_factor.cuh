@@ -52,11 +52,9 @@ constexpr int kTfSlots2 = 624;  // for two
 
 // A list goes on at a piece that was asked for `ago` ticks earlier.  Copies become
 // a group when their tick ends: how many groups may still be under way, or -1 where
-// the copies of this tick, no group yet, have to land as well (rows of a few hundred
-// inputs fill several pieces within a tick).
-__host__ __device__ constexpr int tf_piece_wait(int ago) {
-  return ago >= kTfDelay ? kTfDelay - 1 : ago > 0 ? 0 : -1;
-}
+// all copies have to land, those of this tick, no group yet, among them (rows of a
+// hundred inputs and more fill several pieces within a tick).
+__host__ __device__ constexpr int tf_piece_wait(int ago) { return ago >= kTfDelay ? kTfDelay - 1 : -1; }
 
 struct TileFactor {
   const int4* prog = nullptr;  // null: not available
