@@ -339,12 +339,12 @@ class OSQPEngine:
         solved.  Each slice pays the factorization's latency floor once, so
         few slices; ``first_fraction`` sizes the first slice, whose copy in
         nothing hides; the rest are equal (None: all equal).  Measured on the
-        quadrotor workload (65,536 instances, closed loop, host advance
-        included) with earlier, slower kernels: 4 slices with a 0.15 first
-        slice 109 ms per step, 3 with 0.15 113 ms, 2 with 0.3 127 ms, one 142
-        ms; with the current kernels the default takes 94.5 ms per step (the
-        host advance in ``on_slice``).  Each slice is an ordinary ``solve`` of its instances, so
-        the results equal a one-shot ``solve`` of the whole batch bit for bit.
+        quadrotor workload (65,536 instances, closed loop, the host advance in
+        ``on_slice``): the default of 4 slices with a 0.15 first slice 64.9 ms
+        per step, 4 equal ones 65.7, 5 with 0.15 63.5, 6 64.7, 3 73.0, 2 with
+        0.3 86, one 104.  Each slice is an ordinary ``solve`` of its
+        instances, so the results equal a one-shot ``solve`` of the whole
+        batch bit for bit.
         Inputs should be in pinned memory (pageable tensors still work, without
         the overlap).  ``out`` optionally gives the six host output tensors
         ``(x, z, y, prim_res, dual_res, obj_val)``; otherwise they are
